@@ -474,6 +474,7 @@ static int build_metric(swe_ctx *c, DevMetric<T> &dm)
     v.inv_hxa = T(1.0 / (hx * a));
     v.inv_hx = T(1.0 / hx);
     v.grav = T(c->cfg.grav);
+    CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // the copy above, before the kernel on the context's stream
     k_edge_tables<T><<<(N + 1 + 127) / 128, 128, 0, c->stream>>>(v, c->dims, ej, ef, ea, ord_strip_lines(c->ord));
     CU(c, cudaGetLastError());
     CU(c, cudaStreamSynchronize(c->stream));
@@ -551,6 +552,7 @@ static int build_fused_metric(swe_ctx *c, const MetricView<T> &mv)
     CU(c, cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     // f J^2 per panel: the same values the split kernels use
     CU(c, cudaMemcpy(d + FM_FJ2 * box, mv.fJ2, NPAN * box * sizeof(T), cudaMemcpyDeviceToDevice));
+    CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // before kernels on the context's stream
     if (!encode_rows(&c->tm_metric, d, sizeof(T), P, (int64_t)FM_BOXES * (N + 1 + 2 * MG), fused_box_w(c), c->fth + 8))
         return fail(c, SWE_ECUDA, "TMA tensor map of the fused metric");
     return SWE_OK;
@@ -1009,6 +1011,9 @@ static int alloc_box(swe_ctx *c, void **p)
     size_t bytes = c->box_elems * c->elem;
     if (cudaMalloc(p, bytes) != cudaSuccess) return fail(c, SWE_ENOMEM, "device allocation of %zu bytes failed", bytes);
     CU(c, cudaMemset(*p, 0, bytes));
+    // the context's stream does not block on the default stream: without this wait the clear
+    // could run after an upload there and wipe the uploaded state
+    CU(c, cudaStreamSynchronize(cudaStreamLegacy));
     return SWE_OK;
 }
 
@@ -1113,6 +1118,9 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
     if (cudaHostAlloc((void **)&c->pinned, c->box_elems * c->elem, cudaHostAllocDefault) != cudaSuccess)
         return bail(SWE_ENOMEM);
     std::memset(c->pinned, 0, c->box_elems * c->elem);
+    // every table and cleared buffer in place, whatever stream the context works on next
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return bail(SWE_ECUDA);
     *out = c;
     return SWE_OK;
 }
@@ -2189,6 +2197,7 @@ static int dif_setup(swe_ctx *c)
         if (cudaMalloc(&c->dif_b, h.size() * sizeof(T)) != cudaSuccess)
             return fail(c, SWE_ENOMEM, "diffusion basis allocation failed");
         CU(c, cudaMemcpy(c->dif_b, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+        CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // before kernels on the context's stream
     }
     if (!c->dif && cudaMalloc(&c->dif, 5 * M * DIF_FIELDS * NPAN * box * sizeof(T)) != cudaSuccess)
         return fail(c, SWE_ENOMEM, "diffusion scratch allocation failed");
