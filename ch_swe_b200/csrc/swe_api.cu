@@ -21,6 +21,7 @@
 #include "swe_diff.cuh"
 #include "swe_kernels.cuh"
 #include "swe_launch.cuh"
+#include "swe_one_launch.cuh"
 
 namespace chswe {
 
@@ -269,6 +270,13 @@ struct swe_ctx {
     int fth = 25, focc = 3;
     void *fmet = nullptr;            // FM_BOXES metric boxes of the fused stage (built on first use)
     CUtensorMap tm_metric;           // TMA map of fmet
+    // one-launch stage (swe_onepass.cuh) of the linear Ch 4-2 operator: selected instead of
+    // the split kernels and the fused stage when `one`; (olabel, oocc) is its configuration.
+    // A context of that operator starts with it (`one_default`) until a configuration is set.
+    bool one = false, one_default = false;
+    int olabel = 0, oocc = 0;
+    void *onetab = nullptr;          // OneMetric tables (side lines, edge-vector weights)
+    CUtensorMap tm_one;              // TMA map of fmet with the one-launch stage's tiles
     int *derr = nullptr;             // device error word: a bounded wait in a kernel gave up
     bool launch_miss = false;        // a stage or contravariant launch found no built configuration
     bool graph_members = false;      // the cached graph uses the per-member time steps
@@ -397,6 +405,8 @@ static cudaError_t upload_link_tables()
     if (e == cudaSuccess) e = StageTU<double, 33>::upload_tables(l, q);
     if (e == cudaSuccess) e = FusedTU<float>::upload_tables(l);
     if (e == cudaSuccess) e = FusedTU<double>::upload_tables(l);
+    if (e == cudaSuccess) e = OneTU<float>::upload_tables(l);
+    if (e == cudaSuccess) e = OneTU<double>::upload_tables(l);
     if (e == cudaSuccess) e = GroupTU<float>::upload_tables(l, q);
     if (e == cudaSuccess) e = GroupTU<double>::upload_tables(l, q);
     return e;
@@ -553,13 +563,17 @@ static int build_fused_metric(swe_ctx *c, const MetricView<T> &mv)
     // f J^2 per panel: the same values the split kernels use
     CU(c, cudaMemcpy(d + FM_FJ2 * box, mv.fJ2, NPAN * box * sizeof(T), cudaMemcpyDeviceToDevice));
     CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // before kernels on the context's stream
-    if (!encode_rows(&c->tm_metric, d, sizeof(T), P, (int64_t)FM_BOXES * (N + 1 + 2 * MG), fused_box_w(c), c->fth + 8))
-        return fail(c, SWE_ECUDA, "TMA tensor map of the fused metric");
     return SWE_OK;
 }
 
 // The fused stage serves the linear operator on the Ch grid in SBP 4-2.
 static bool fused_supported(const swe_ctx *c) { return !c->adv && !c->ah && c->ord == 42; }
+
+static int ensure_fused_metric(swe_ctx *c)
+{
+    if (c->fmet) return SWE_OK;
+    return c->elem == 8 ? build_fused_metric<double>(c, c->m64.v) : build_fused_metric<float>(c, c->m32.v);
+}
 
 static bool fused_cfg_built(const swe_ctx *c, int th, int occ)
 {
@@ -580,19 +594,65 @@ static int select_fused(swe_ctx *c, int th, int occ)
     dim3 g;
     if (!fused_supported(c) || !fused_cfg_built(c, th, occ) || !fused_grid(c->cfg.N, c->cfg.n_members, th, g))
         return fail(c, SWE_EINVAL, "fused stage configuration (%d, %d) is not available for this context", th, occ);
-    const bool retile = c->fth != th;
+    if (int rc = ensure_fused_metric(c)) return rc;
     c->fth = th;
     c->focc = occ;
-    c->fused = true;
-    if (!c->fmet) {
-        int rc = c->elem == 8 ? build_fused_metric<double>(c, c->m64.v) : build_fused_metric<float>(c, c->m32.v);
-        if (rc) { c->fused = false; return rc; }
-    } else if (retile &&
-               !encode_rows(&c->tm_metric, c->fmet, c->elem, c->dims.P,
-                            (int64_t)FM_BOXES * (c->cfg.N + 1 + 2 * MG), fused_box_w(c), th + 8)) {
+    if (!encode_rows(&c->tm_metric, c->fmet, c->elem, c->dims.P, (int64_t)FM_BOXES * (c->cfg.N + 1 + 2 * MG), fused_box_w(c),
+                     th + 8)) {
         c->fused = false;
         return fail(c, SWE_ECUDA, "TMA tensor map of the fused metric");
     }
+    c->fused = true;
+    return SWE_OK;
+}
+
+// The one-launch stage's tables: the metric along the panel sides (from fmet, so the same
+// values) and the dense weights of the edge vectors.
+template <class T>
+static int build_one_tables(swe_ctx *c)
+{
+    constexpr int VW = OV<T>::W, NW = XROW_OPS * ONE_EDGES * ONE_TAPS * VW;
+    const size_t ns = (size_t)4 * ONE_LINES * (c->cfg.N + 1), so = (NW + 31) / 32 * 32;
+    std::vector<double> w(NW);
+    one_edge_table(c->cfg.N, VW, w.data());
+    std::vector<T> wt(w.begin(), w.end());
+    T *d = nullptr;
+    if (cudaMalloc(&d, (so + ns) * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "stage table allocation failed");
+    c->onetab = d;
+    CU(c, cudaMemcpy(d, wt.data(), NW * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, cudaStreamSynchronize(cudaStreamLegacy));
+    OneTU<T>::tables((const T *)c->fmet, d + so, c->dims, c->stream);
+    CU(c, cudaGetLastError());
+    CU(c, cudaStreamSynchronize(c->stream));
+    return SWE_OK;
+}
+template <class T>
+static OneMetric<T> one_metric(const swe_ctx *c, const MetricView<T> &mv)
+{
+    constexpr int NW = XROW_OPS * ONE_EDGES * ONE_TAPS * OV<T>::W;
+    const T *d = (const T *)c->onetab;
+    return OneMetric<T>{d + (NW + 31) / 32 * 32, d, mv.ea, mv.ef, mv.qb, mv.qt, mv.ql, mv.qr, mv.inv_hxa, mv.inv_hx, mv.grav};
+}
+
+// Select the one-launch stage with configuration (label, occ).
+static int select_one(swe_ctx *c, int label, int occ)
+{
+    OneGrid og;
+    int bw = 0, bh = 0;
+    const bool f64 = c->elem == 8;
+    const bool built = f64 ? OneTU<double>::box(label, occ, bw, bh) && OneTU<double>::grid(label, occ, c->cfg.N, c->cfg.n_members, og)
+                           : OneTU<float>::box(label, occ, bw, bh) && OneTU<float>::grid(label, occ, c->cfg.N, c->cfg.n_members, og);
+    if (!fused_supported(c) || c->cstag || !built)
+        return fail(c, SWE_EINVAL, "one-launch stage configuration (%d, %d) is not available for this context", label, occ);
+    if (int rc = ensure_fused_metric(c)) return rc;
+    if (!c->onetab)
+        if (int rc = f64 ? build_one_tables<double>(c) : build_one_tables<float>(c)) return rc;
+    c->one = false;
+    if (!encode_rows(&c->tm_one, c->fmet, c->elem, c->dims.P, (int64_t)FM_BOXES * (c->cfg.N + 1 + 2 * MG), bw, bh))
+        return fail(c, SWE_ECUDA, "TMA tensor map of the stage metric");
+    c->olabel = label;
+    c->oocc = occ;
+    c->one = true;
     return SWE_OK;
 }
 
@@ -998,7 +1058,7 @@ static void free_ctx(swe_ctx *c)
     cudaFree(c->fl); cudaFree(c->adt); cudaFree(c->fs); cudaFree(c->vh); cudaFree(c->ones); cudaFree(c->hb);
     cudaFree(c->ah64.base); cudaFree(c->ah32.base); cudaFree(c->qa); cudaFree(c->negones);
     cudaFree(c->dif); cudaFree(c->dif_b);
-    cudaFree(c->fmet); cudaFree(c->derr); cudaFree(c->hs); cudaFree(c->cmet);
+    cudaFree(c->fmet); cudaFree(c->onetab); cudaFree(c->derr); cudaFree(c->hs); cudaFree(c->cmet);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     if (c->side) cudaStreamDestroy(c->side);
@@ -1019,6 +1079,28 @@ static int alloc_box(swe_ctx *c, void **p)
 
 template <class T>
 static cudaError_t stage_smem_optin();
+
+// The one-launch configuration a linear Ch 4-2 context starts with; tile 0: the split
+// kernels.  Cubes below 16 cells keep the split kernels and their twelve launches a step,
+// which swe_launch_count reports there.  FP32 starts with the large tiles (measured per RK4
+// step at C24 / C48 / C96 / C192: 24 / 27 / 28 / 33 us against 85 / 75 / 80 / 86 us split).
+// FP64: the one-block-per-SM tiles where the grid fits one wave (C24 / C48 / C96: 23 / 24 /
+// 33 against 97 / 91 / 96 us split); where it does not, their advantage shrinks (C192: 83
+// against 102 us) and small cubes with many members are faster split (64 x C48: 496 against
+// 425 us: every tile holds a panel corner).
+template <class T>
+static KernelCfg one_default_cfg(int N, int members)
+{
+    OneGrid og;
+    const KernelCfg none{0, 0, 0};
+    if (N < 16) return none;
+    if (sizeof(T) == 4) return OneTU<T>::grid(33, 2, N, members, og) ? KernelCfg{33, 2, 3} : none;
+    if (N < 128 && members > 4) return none;
+    for (int label : {25, 33})
+        if (OneTU<T>::grid(label, 1, N, members, og) && (og.g.x * og.g.y * og.g.z <= 148 || label == 33))
+            return KernelCfg{label, 1, 3};
+    return OneTU<T>::grid(17, 2, N, members, og) ? KernelCfg{17, 2, 3} : none;
+}
 
 extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
 {
@@ -1113,6 +1195,13 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
                 for (cudaEvent_t *e : {&c->ev_fork, &c->ev_havg, &c->ev_co2, &c->ev_side})
                     if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return bail(SWE_ECUDA);
             }
+        }
+    }
+    if (fused_supported(c) && !c->cstag) {
+        const KernelCfg k = c->elem == 8 ? one_default_cfg<double>(N, cfg->n_members) : one_default_cfg<float>(N, cfg->n_members);
+        if (k.tile) {
+            if ((rc = select_one(c, k.tile, k.occ)) != SWE_OK) return bail(rc);
+            c->one_default = true;
         }
     }
     if (cudaHostAlloc((void **)&c->pinned, c->box_elems * c->elem, cudaHostAllocDefault) != cudaSuccess)
@@ -1426,6 +1515,7 @@ static cudaError_t stage_smem_optin()
     if (e == cudaSuccess) e = StageTU<T, 25>::optin();
     if (e == cudaSuccess) e = StageTU<T, 33>::optin();
     if (e == cudaSuccess) e = FusedTU<T>::optin();
+    if (e == cudaSuccess) e = OneTU<T>::optin();
     if (e == cudaSuccess) e = GroupTU<T>::optin();
     if (e == cudaSuccess) e = set_carveout(k_edge<T, 42>);
     if (e == cudaSuccess) e = set_carveout(k_edge<T, 21>);
@@ -1516,6 +1606,25 @@ static bool enqueue_fused(swe_ctx *c, const void *yin, void *v0, void *y1, void 
     return true;
 }
 
+// One RK stage as one launch.
+template <class T>
+static bool enqueue_one(swe_ctx *c, const void *yin, void *v0, void *y1, void *acc, float *cmp, int mode, double dt,
+                        const double *dtm, const double *Hm, const MetricView<T> &mv)
+{
+    const int M = c->cfg.n_members, N = c->cfg.N;
+    int bw, bh;
+    CUtensorMap tmY;
+    if (!OneTU<T>::box(c->olabel, c->oocc, bw, bh) ||
+        !encode_rows(&tmY, yin, sizeof(T), c->dims.P, (int64_t)M * 3 * NPAN * (N + 1 + 2 * MG), bw, bh))
+        return false;
+    StageArgs a{mode, dt, Hm, dtm, nullptr, nullptr, nullptr};
+    if (!OneTU<T>::stage(c->olabel, c->oocc, M, tmY, c->tm_one, (const T *)yin, (T *)v0, (T *)y1, (T *)acc, (T *)cmp, c->dims,
+                         one_metric<T>(c, mv), a, c->derr, c->stream))
+        return false;
+    c->launches++;
+    return true;
+}
+
 // The advective tendencies (k_advt): tiles of 32 x 16 xy points from C128 on, 32 x 8
 // below (where taller tiles would leave fewer blocks than SMs).
 template <class T>
@@ -1549,6 +1658,12 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
         return;
     }
     if (!c->adv) {
+        if (c->one) {
+            if (enqueue_one<T>(c, yin, v0, y1, acc, cmp, mode, dt, dtm, c->Hm, mv)) return;
+            // a tensor map that cannot be encoded: the split kernels take over
+            c->one = false;
+            c->err = "one-launch stage unavailable (TMA tensor map); using the split stage kernels";
+        }
         if (c->fused) {
             if (enqueue_fused<T>(c, yin, v0, y1, acc, cmp, mode, dt, dtm, mv)) return;
             // a tensor map that cannot be encoded: the split kernels take over
@@ -1876,7 +1991,8 @@ extern "C" int swe_group_create(swe_ctx *const *ctxs, int n, swe_group **out)
             return fail(c0, SWE_EINVAL, "group: context %d has another device or precision than context 0", k);
         if (c->adv || c->ah || c->cstag || c->ord != 42)
             return fail(c0, SWE_EINVAL, "group: context %d is not the linear operator on Ch in SBP 4-2", k);
-        if (c->fused || c->tile != c0->tile || c->occ != c0->occ || c->runs != c0->runs)
+        // a context on its default stage joins with its split configuration
+        if (c->fused || (c->one && !c->one_default) || c->tile != c0->tile || c->occ != c0->occ || c->runs != c0->runs)
             return fail(c0, SWE_EINVAL, "group: context %d has another kernel configuration than context 0 "
                         "(the contexts share one split configuration)", k);
     }
@@ -1999,7 +2115,7 @@ extern "C" int swe_group_rk4_steps_members(swe_group *g, swe_stvec *const *state
             if (!(dt[k][m] >= 0.0) || !std::isfinite(dt[k][m]))
                 return gfail(g, SWE_EINVAL, "group: context %d member %d: time step %g (need finite, >= 0)", k, m,
                              dt[k][m]);
-        if (c->fused || c->tile != g->tile || c->occ != g->occ || c->runs != g->runs)
+        if (c->fused || (c->one && !c->one_default) || c->tile != g->tile || c->occ != g->occ || c->runs != g->runs)
             return gfail(g, SWE_EINVAL, "group: context %d changed its kernel configuration", k);
     }
     if (nsteps == 0) return SWE_OK;
@@ -3347,6 +3463,15 @@ static void timed_stage(swe_ctx *c, const MetricView<T> &mv, const void *yin, vo
                         double dt, cudaEvent_t e0, cudaEvent_t e1, cudaEvent_t e2, cudaEvent_t e3)
 {
     const int M = c->cfg.n_members;
+    if (c->one) {
+        // one-launch stage: all of its time is the stage kernel's
+        cudaEventRecord(e0, c->stream);
+        cudaEventRecord(e1, c->stream);
+        cudaEventRecord(e2, c->stream);
+        if (!enqueue_one<T>(c, yin, v0, y1, c->acc, cmp, mode, dt, nullptr, c->Hm, mv)) c->launch_miss = true;
+        cudaEventRecord(e3, c->stream);
+        return;
+    }
     if (c->fused) {
         // fused stage: the edge-strip kernel, the edge sync, the tiles
         const FusedMetric<T> fm{(const T *)c->fmet, mv.inv_hxa, mv.inv_hx, mv.grav};
@@ -3657,18 +3782,28 @@ static void set_cfg(swe_ctx *c, int tile, int occ, int runs)
 }
 
 // runs 0 / 1: the split stage kernels (tile, blocks per SM, stencil runs); runs 2: the
-// fused stage with tiles of at most `tile` rows (17, 25 or 33) and FUSED_TW columns.
+// fused stage with tiles of at most `tile` rows (17, 25 or 33) and FUSED_TW columns; runs 3:
+// the one-launch stage with tiles of at most `tile` rows.
 static int apply_cfg(swe_ctx *c, int tile, int occ, int runs)
 {
+    if (runs == 3) {
+        const bool changed = !c->one || c->olabel != tile || c->oocc != occ;
+        int rc = select_one(c, tile, occ);
+        if (rc) return rc;
+        if (changed) drop_graph(c);
+        c->fused = c->one_default = false;
+        return SWE_OK;
+    }
     if (runs == 2) {
-        const bool changed = !c->fused || c->fth != tile || c->focc != occ;
+        const bool changed = c->one || !c->fused || c->fth != tile || c->focc != occ;
         int rc = select_fused(c, tile, occ);
         if (rc) return rc;
         if (changed) drop_graph(c);
+        c->one = c->one_default = false;
         return SWE_OK;
     }
-    if (c->fused) drop_graph(c);
-    c->fused = false;
+    if (c->fused || c->one) drop_graph(c);
+    c->fused = c->one = c->one_default = false;
     set_cfg(c, tile, occ, runs);
     return SWE_OK;
 }
@@ -3682,14 +3817,14 @@ extern "C" int swe_set_tile(swe_ctx *c, int tile)
 extern "C" int swe_get_tile(const swe_ctx *c, int *tile)
 {
     if (!c || !tile) return SWE_EINVAL;
-    *tile = c->fused ? c->fth : c->tile;
+    *tile = c->one && !c->one_default ? c->olabel : (c->fused ? c->fth : c->tile);
     return SWE_OK;
 }
 
 extern "C" int swe_set_kernel_config(swe_ctx *c, int tile, int blocks_per_sm, int runs)
 {
     if (!c) return SWE_EINVAL;
-    if (runs == 2) return apply_cfg(c, tile, blocks_per_sm, runs);
+    if (runs == 2 || runs == 3) return apply_cfg(c, tile, blocks_per_sm, runs);
     if (!valid_cfg(c->ord, tile, blocks_per_sm, runs)) return SWE_EINVAL;
     return apply_cfg(c, tile, blocks_per_sm, runs);
 }
@@ -3697,6 +3832,12 @@ extern "C" int swe_set_kernel_config(swe_ctx *c, int tile, int blocks_per_sm, in
 extern "C" int swe_get_kernel_config(const swe_ctx *c, int *tile, int *blocks_per_sm, int *runs)
 {
     if (!c || !tile || !blocks_per_sm || !runs) return SWE_EINVAL;
+    if (c->one) {
+        *tile = c->olabel;
+        *blocks_per_sm = c->oocc;
+        *runs = 3;
+        return SWE_OK;
+    }
     if (c->fused) {
         *tile = c->fth;
         *blocks_per_sm = c->focc;
@@ -3754,8 +3895,9 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
     swe_stvec *v = nullptr;
     int rc = swe_stvec_create(c, &v);
     if (rc) return rc;
-    const int keep_tile = c->fused ? c->fth : c->tile, keep_occ = c->fused ? c->focc : c->occ,
-              keep_runs = c->fused ? 2 : c->runs;
+    const int keep_tile = c->one ? c->olabel : (c->fused ? c->fth : c->tile),
+              keep_occ = c->one ? c->oocc : (c->fused ? c->focc : c->occ), keep_runs = c->one ? 3 : (c->fused ? 2 : c->runs);
+    const bool keep_default = c->one_default;
     double ms[3] = {1e300, 1e300, 1e300};
     int best_t = keep_tile, best_o = keep_occ, best_r = keep_runs;
     double best_ms = 1e300;
@@ -3777,6 +3919,14 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
             CHSWE_FUSED_CFGS_D(CHSWE_FADD)
         }
 #undef CHSWE_FADD
+        // and the one-launch stage's
+#define CHSWE_OADD(LABEL, XL, TH, OCC, REGS) all.push_back(KernelCfg{LABEL, OCC, 3});
+        if (c->elem == 4) {
+            CHSWE_ONE_CFGS_F(CHSWE_OADD)
+        } else {
+            CHSWE_ONE_CFGS_D(CHSWE_OADD)
+        }
+#undef CHSWE_OADD
     }
     for (size_t k = 0; k < all.size() && rc == SWE_OK; k++) {
         const KernelCfg kc = all[k];
@@ -3823,7 +3973,11 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
     if (e1) cudaEventDestroy(e1);
     swe_stvec_destroy(v);
     drop_graph(c);
-    if (rc != SWE_OK) { apply_cfg(c, keep_tile, keep_occ, keep_runs); return rc; }
+    if (rc != SWE_OK) {
+        apply_cfg(c, keep_tile, keep_occ, keep_runs);
+        c->one_default = keep_default;
+        return rc;
+    }
     if ((rc = apply_cfg(c, best_t, best_o, best_r)) != SWE_OK) return rc;
     TuneEntry te{key, best_t, best_o, best_r, {ms[0], ms[1], ms[2]}, best_b};
     g_tuned.push_back(te);

@@ -1,0 +1,113 @@
+"""The one-launch stage of the linear Ch operator (SBP 4-2) against the CPU FP64 oracle.
+
+Every tile computes the neighbour panels' boundary values it needs itself, so the cube
+sizes put the panel's far edge at every position within a vector of points (four FP32, two
+FP64), with one, two and several tiles per direction.  Random states: the duplicated edge
+vertices and both winds disagree across the panels.  Tolerances as for the other stage
+kernels: FP64 within 1e-12 relative (max-norm) of the oracle, FP32 within 1e-5.
+"""
+import numpy as np
+import pytest
+
+from ch_swe_b200._lib import SweError
+from tests.conftest import gpu_available
+
+pytestmark = pytest.mark.gpu
+
+LIN = {"swm_operator_type": "linear_swm_operator", "h_mean": 1000.0}
+CFGS = [("fp64", c) for c in ((17, 2, 3), (25, 1, 3), (33, 1, 3))] + [("fp32", c) for c in ((17, 2, 3), (25, 1, 3), (25, 2, 3), (33, 2, 3))]
+RTOL = {"fp64": 1e-12, "fp32": 1e-5}
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu(lib_built, oracle_built):
+    if not gpu_available():
+        pytest.fail("no CUDA device: the -m gpu tests need a B200")
+
+
+def rel(a, b):
+    return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
+
+
+def random_state(N, seed):
+    from ch_swe_b200 import state_shapes
+    rng = np.random.default_rng(seed)
+    return tuple(rng.standard_normal(s) for s in state_shapes(N))
+
+
+@pytest.mark.parametrize("precision,cfg", CFGS)
+@pytest.mark.parametrize("N", [8, 9, 10, 11, 16, 21, 23, 24, 31, 32, 33, 34, 46, 48, 65, 79])
+def test_apply_matches_oracle(precision, cfg, N):
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator
+    from oracle.oracle import Oracle
+    h, u, v = random_state(N, 900 + N)
+    axis = (0.3, -0.5, 0.8)
+    ref = Oracle(N, h_mean=1000.0, axis=axis).apply(h, u, v)
+    dom = create_domain(N, precision=precision, h_mean=1000.0, rotation_axis=axis)
+    if cfg[1] == 1 and N <= 24:
+        # a block that touches four sides does not fit the register file with these configurations
+        try:
+            dom.kernel_config = cfg
+        except SweError:
+            return
+    dom.kernel_config = cfg
+    assert dom.kernel_config == cfg
+    op = create_swm_operator(dom.grav, LIN, dom)
+    x, y = create_stvec_swm(dom).upload(h, u, v), create_stvec_swm(dom)
+    op.apply(y, x, dom)
+    dom.synchronize()
+    for g, r, name in zip(y.download(), ref, "huv"):
+        assert rel(g, r) < RTOL[precision], (name, rel(g, r))
+    dom.destroy()
+
+
+@pytest.mark.parametrize("precision,cfg", CFGS)
+def test_rk4_members_match_the_split_stage(precision, cfg):
+    """Steps with a time step per member (one frozen) and a mean depth per member agree with
+    the split kernels to rounding; the zero margins and the frozen member stay as they were."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    N, M = 37, 3
+    states = [random_state(N, 40 + k) for k in range(M)]
+    stack = [np.stack([s[f] for s in states]) for f in range(3)]
+    dts = np.array([300.0, 0.0, 150.0])
+    out = []
+    for c in (cfg, (25, 2, 0)):
+        dom = create_domain(N, precision=precision, n_members=M, h_mean=1000.0)
+        dom.kernel_config = c
+        op = create_swm_operator(dom.grav, LIN, dom)
+        op.set_member_h_mean(2, 700.0)
+        st = create_stvec_swm(dom).upload(*stack, member=None)
+        create_timescheme(st, "rk4").steps_members(st, op, dts, 11)
+        dom.synchronize()
+        out.append(st.download(member=None))
+        dom.destroy()
+    for f in range(3):
+        assert rel(out[0][f], out[1][f]) < RTOL[precision]
+        assert np.array_equal(out[0][f][1], stack[f][1].astype(np.float32 if precision == "fp32" else np.float64))
+
+
+def test_default_stage_matches_oracle_and_joins_a_group():
+    """A linear context that sets no configuration runs the one-launch stage; a group takes it
+    with its split configuration."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    from ch_swe_b200.swm import create_group
+    from oracle.oracle import Oracle
+    N, dt = 100, 200.0
+    o = Oracle(N, h_mean=1000.0)
+    ic = o.gaussian(lam0=0.7, phi0=0.2, d0=0.2)
+    ref = o.rk4(*ic, dt, 3)
+    dom = create_domain(N, h_mean=1000.0)
+    assert dom.kernel_config[2] == 3 and dom.tile == 33
+    op = create_swm_operator(dom.grav, LIN, dom)
+    st = create_stvec_swm(dom).upload(*ic)
+    create_timescheme(st, "rk4").steps(st, op, dom, dt, 3)
+    for g, r in zip(st.download(), ref):
+        assert rel(g, r) < 1e-12
+    st.upload(*ic)
+    g = create_group([dom])
+    g.steps_members([st], [np.array([dt])], 3)
+    g.synchronize()
+    for a, r in zip(st.download(), ref):
+        assert rel(a, r) < 1e-12
+    g.destroy()
+    dom.destroy()
