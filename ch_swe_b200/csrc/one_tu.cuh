@@ -17,16 +17,10 @@ namespace chswe {
 static inline bool one_fits(int warps, int regs) { return (warps + 3) / 4 * 32 * regs <= 16384; }
 
 template <class T, int XL, int TH, int REGS>
-static cudaError_t one_optin_modes()
+static cudaError_t one_optin()
 {
-    const int sb = (int)OneLayout<T, XL, TH>::bytes(4);
-    void (*f[5])(CUtensorMap, CUtensorMap, const T *, T *, T *, T *, T *, Dims, OneMetric<T>, StageArgs, int *) = {
-        k_onepass<T, XL, TH, REGS, 0>, k_onepass<T, XL, TH, REGS, 1>, k_onepass<T, XL, TH, REGS, 2>,
-        k_onepass<T, XL, TH, REGS, 3>, k_onepass<T, XL, TH, REGS, 4>};
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < 5 && e == cudaSuccess; k++)
-        e = cudaFuncSetAttribute(f[k], cudaFuncAttributeMaxDynamicSharedMemorySize, sb);
-    return e;
+    return cudaFuncSetAttribute(k_onepass<T, XL, TH, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)OneLayout<T, XL, TH>::bytes(4));
 }
 
 template <class T>
@@ -34,7 +28,7 @@ cudaError_t OneTU<T>::optin()
 {
     cudaError_t e = cudaSuccess;
 #define CHSWE_O(LABEL, XL, TH, OCC, REGS) \
-    if (e == cudaSuccess) e = one_optin_modes<T, XL, TH, REGS>();
+    if (e == cudaSuccess) e = one_optin<T, XL, TH, REGS>();
     CHSWE_ONE_EACH(CHSWE_O)
 #undef CHSWE_O
     return e;
@@ -73,24 +67,14 @@ bool OneTU<T>::stage(int label, int occ, int members, const CUtensorMap &tmY, co
 {
     OneGrid og;
     if (!grid(label, occ, d.N, members, og)) return false;
-#define CHSWE_M(XL, TH, REGS, M)                                                                                      \
-    launch_k(k_onepass<T, XL, TH, REGS, M>, og.g, dim3(OneLayout<T, XL, TH>::NM + og.sides * ONE_BAND), \
-             OneLayout<T, XL, TH>::bytes(og.sides), \
-             st, tmY, tmM, y, v0, y1, acc, cmp, d, om, a, err)
-#define CHSWE_O(LABEL, XL, TH, OCC, REGS)                          \
-    if (label == LABEL && occ == OCC) {                      \
-        switch (a.mode) {                                    \
-        case 0: CHSWE_M(XL, TH, REGS, 0); break;              \
-        case 1: CHSWE_M(XL, TH, REGS, 1); break;              \
-        case 2: CHSWE_M(XL, TH, REGS, 2); break;              \
-        case 3: CHSWE_M(XL, TH, REGS, 3); break;              \
-        default: CHSWE_M(XL, TH, REGS, 4); break;             \
-        }                                                    \
-        return true;                                         \
+#define CHSWE_O(LABEL, XL, TH, OCC, REGS)                                                                            \
+    if (label == LABEL && occ == OCC) {                                                                              \
+        launch_k(k_onepass<T, XL, TH, REGS>, og.g, dim3(OneLayout<T, XL, TH>::NM + og.sides * ONE_BAND),             \
+                 OneLayout<T, XL, TH>::bytes(og.sides), st, tmY, tmM, y, v0, y1, acc, cmp, d, om, og.t, a, err);     \
+        return true;                                                                                                 \
     }
     CHSWE_ONE_EACH(CHSWE_O)
 #undef CHSWE_O
-#undef CHSWE_M
     return false;
 }
 

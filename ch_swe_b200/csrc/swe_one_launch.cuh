@@ -76,8 +76,14 @@ static inline void one_edge_table(int N, int VW, double *we)
 #define CHSWE_ONE_CFGS_F(X) X(17, 16, 16, 2, 64) X(25, 16, 25, 1, 80) X(25, 10, 22, 2, 64) X(33, 10, 30, 2, 64)
 #define CHSWE_ONE_CFGS_D(X) X(17, 16, 16, 2, 64) X(25, 16, 22, 1, 96) X(33, 16, 30, 1, 80)
 
+// Balanced tiles: the first rx (ry) tiles hold qx + 1 vectors (qy + 1 rows), the others qx (qy).
+struct OneTiles {
+    int qx, rx, qy, ry;
+};
+
 struct OneGrid {
     dim3 g;
+    OneTiles t;
     int sides;   // panel sides a tile can touch
 };
 
@@ -103,6 +109,7 @@ static inline bool one_grid(int N, int members, int xl, int th, int occ, OneGrid
     }
     if (!best) return false;
     og.g = dim3(gx, best, NPAN * members);
+    og.t = OneTiles{nv / gx, nv % gx, n / best, n % best};
     og.sides = (gx == 1 ? 2 : 1) + (best == 1 ? 2 : 1);
     return true;
 }

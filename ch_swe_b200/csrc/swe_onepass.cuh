@@ -250,10 +250,12 @@ __device__ __forceinline__ T one_across(const OneRaw<T> &r, int s, T Ch)
 //   MODE 0: out = A(y);   1: Y1 = V0 + dt/2 k, ACC = dt/6 k;   2: Y1 = V0 + dt/2 k, ACC += dt/3 k;
 //   3: Y1 = V0 + dt k, ACC += dt/3 k;   4: V0 += ACC + dt/6 k (FP32: Kahan with compensation CMP)
 // Mode 1 takes V0 from the windows: its stage input is V0.
-template <class T, int XL, int TH, int REGS, int MODE>
+// The mode is an argument: one kernel serves the four stages of a step, whose code then
+// stays in the instruction caches from one stage to the next.
+template <class T, int XL, int TH, int REGS>
 __global__ void __maxnreg__(REGS)
     k_onepass(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmM, const T *__restrict__ Yin,
-              T *V0, T *Y1, T *ACC, T *CMP, Dims d, OneMetric<T> om, StageArgs a, int *err)
+              T *V0, T *Y1, T *ACC, T *CMP, Dims d, OneMetric<T> om, OneTiles ot, StageArgs a, int *err)
 {
     using L = OneLayout<T, XL, TH>;
     using SB = SbpOrder<42>;
@@ -274,10 +276,10 @@ __global__ void __maxnreg__(REGS)
     const int N = d.N, n = N + 1, P = d.P;
     const int t = blockIdx.z % NPAN, mem = blockIdx.z / NPAN;
     if (member_frozen(a.dtm, mem)) return;
-    const int NV = (n + VW - 1) / VW;
-    const int v0 = (blockIdx.x * NV) / gridDim.x, v1 = ((blockIdx.x + 1) * NV) / gridDim.x;
+    const int NV = (n + VW - 1) / VW, bx = blockIdx.x, by = blockIdx.y;
+    const int v0 = bx * ot.qx + min(bx, ot.rx), v1 = v0 + ot.qx + (bx < ot.rx);
     const int i0 = 1 + VW * v0, i1 = min(1 + VW * v1, n + 1);
-    const int j0 = 1 + (blockIdx.y * n) / gridDim.y, j1 = 1 + ((blockIdx.y + 1) * n) / gridDim.y;
+    const int j0 = 1 + by * ot.qy + min(by, ot.ry), j1 = j0 + ot.qy + (by < ot.ry);
     const int tid = threadIdx.x;
     const int rows = N + 1 + 2 * MG;
     // slot offset of point (i, j)
@@ -363,6 +365,21 @@ __global__ void __maxnreg__(REGS)
             one_rowsel(2, al, N, bC, w);
 #pragma unroll
             for (int m = 0; m < 5; m++) wC[m] = __ldg(gx + w + m);
+        }
+        // a panel corner: the third panel is the neighbour across s2 (this thread's other side); the
+        // signs of the second SATs
+        const bool corner = al == 1 || al == n;
+        const int s2 = lr ? (al == 1 ? SIDE_B : SIDE_T) : SIDE_L;
+        T sn2 = T(0), sgx = T(0), sgy = T(0);
+        bool y1 = false, y21 = false;
+        if (corner && lr && b < ONE_BAND) {
+            const Link K2 = c_link[t][s2];
+            const int kc = s == SIDE_L ? 1 : n, y2 = K2.rev ? n + 1 - kc : kc;
+            y1 = y == 1;
+            y21 = y2 == 1;
+            sn2 = T(K2.sn);
+            sgx = T(c_link[K.nb][nlr ? (y1 ? SIDE_B : SIDE_T) : (y1 ? SIDE_L : SIDE_R)].sn);
+            sgy = T(c_link[K2.nb][K2.nside <= SIDE_R ? (y21 ? SIDE_B : SIDE_T) : (y21 ? SIDE_L : SIDE_R)].sn);
         }
         // zeros beyond the band, which taps of weight zero read
         for (int q = b; q < L::BAND; q += ONE_BAND) bd[q] = T(0);
@@ -471,7 +488,6 @@ __global__ void __maxnreg__(REGS)
         T up, vp;
         one_vec(ro, s, fo, up, vp);
         const T dn = one_across(rn, K.nside, T(K.sn) * ro.C) + rn.T2, dv = one_across(ro, s, T(K.sn) * rn.C) + ro.T2;
-        const bool corner = al == 1 || al == n;
         if (vx && !full) {
             // beyond the tile only the component along the side is read
             if (lr) sVP[SI(kk, ll)] = T(0.5) * (vp + vh);
@@ -491,20 +507,13 @@ __global__ void __maxnreg__(REGS)
             }
             nbar_sync(BAR_CORN, nband);
             if (full && corner && lr) {
-                // the third panel: the neighbour across the bottom or top side through this corner
-                const int s2 = al == 1 ? SIDE_B : SIDE_T;
-                const Link K2 = c_link[t][s2];
                 const T *c = sm + L::CORN + (s2 * 2 + (kk == 1 ? 0 : 1)) * 8;
-                const int y2 = K2.rev ? n + 1 - kk : kk;
                 const T satc = T(SB::SATC);
                 // the second SAT at the corner, of every copy: own across s2 (its normal component next
                 // to the corner is the tangential one of side s), the neighbour's toward the third panel
                 // and the third panel's toward the neighbour
-                const int sx = K.nside <= SIDE_R ? (y == 1 ? SIDE_B : SIDE_T) : (y == 1 ? SIDE_L : SIDE_R);
-                const int sy = K2.nside <= SIDE_R ? (y2 == 1 ? SIDE_B : SIDE_T) : (y2 == 1 ? SIDE_L : SIDE_R);
-                const T jo = satc * (ro.K - T(K2.sn) * c[2]), jx = satc * (rn.K - T(c_link[K.nb][sx].sn) * c[3]),
-                        jy = satc * (c[3] - T(c_link[K2.nb][sy].sn) * rn.K);
-                const T d0 = al == 1 ? dv + jo : dv - jo, d1 = y == 1 ? dn + jx : dn - jx, d2 = y2 == 1 ? c[4] + jy : c[4] - jy;
+                const T jo = satc * (ro.K - sn2 * c[2]), jx = satc * (rn.K - sgx * c[3]), jy = satc * (c[3] - sgy * rn.K);
+                const T d0 = al == 1 ? dv + jo : dv - jo, d1 = y1 ? dn + jx : dn - jx, d2 = y21 ? c[4] + jy : c[4] - jy;
                 const T sdiv = (d0 * om.inv_hx * eao + d1 * om.inv_hx * ean + d2 * om.inv_hx * c[6]) / T(3);
                 sUP[SI(kk, ll)] = (up + uh + c[0] + qs * vh) / T(3);
                 sVP[SI(kk, ll)] = (vp + vh + c[1] + c[5] * c[0]) / T(3);
@@ -618,115 +627,129 @@ __global__ void __maxnreg__(REGS)
             put(sVP + o, r);
         }
     }
-    // ---- RK4 operands of this thread's points, in flight across the barrier
-    constexpr bool LV = MODE >= 2, LA = MODE >= 2, LC = (sizeof(T) == 4) && MODE == 4;
+    // ---- RK4 operands of this thread's points, in flight across the barrier; in mode 1 V0 is the
+    // stage input, in the windows
+    const int mode = a.mode;
     const int j = j0 + ty;
     const bool work = in_tile && j < j1;
+    const int so = SI(k, j);
     const int64_t po = (int64_t)mem * d.ms + (int64_t)t * d.ps + box_off32(P, k, j);
     const int64_t fs = d.fs;
-    V pv[LV ? 3 : 1]{}, pa[LA ? 3 : 1]{};
-    if constexpr (LV || LA) {
-        if (work) {
+    V pv[3]{}, pa[3]{}, kh, ku, kv;
+    if (work) {
+        if (mode >= 2) {
 #pragma unroll
             for (int f = 0; f < 3; f++) {
                 pv[f] = ov_ld(V0 + po + f * fs);
                 pa[f] = ov_ld(ACC + po + f * fs);
             }
         }
+        // the parts that need no boundary value: divergence and gradient (without the SAT's
+        // neighbour terms)
+        {
+            const V dx = one_x<1>(sJUT + so, ve, ec, we), ia = ov_ld(siJa + so),
+                    dy = one_y<1, false, SW>(sJVT + SI(k, 0), (const T *)nullptr, j, n, xr);
+#pragma unroll
+            for (int e = 0; e < VW; e++) kh.a[e] = (dx.a[e] * om.inv_hx + dy.a[e] * om.inv_hx) * ia.a[e];
+        }
+        ku = one_x<3>(sH + so, ve, ei, we);
+        kv = ov_zero<T, VW>();
+        if (j <= N) kv = one_y<3, false, SW>(sH + SI(k, 0), (const T *)nullptr, j, N, xr);
     }
     if (touch) nbar_sync(BAR_BND, NM + nband);
     else nbar_sync(BAR_MAIN, NM);
     if (!work) return;
 
-    // ---- P4: divergence, gradient, Coriolis at the tile's points and the RK4 update, field by field
-    const int so = SI(k, j);
-    const bool edgecol = k <= 1 || k + VW > n;
-    // RK4 update of one field; elements beyond the field's extent hold zeros and stay zero
-    auto update = [&](int f, const V &kk) {
-        const int64_t of = po + f * fs;
-        V r, q;
-        if constexpr (MODE == 0) {
-            ov_st(Y1 + of, kk);
-        } else if constexpr (MODE <= 3) {
-            const T ca = (MODE == 3) ? dt : T(0.5) * dt;
-            const T cb = (MODE == 1) ? dt / T(6) : dt / T(3);
-            const V v = LV ? pv[LV ? f : 0] : ov_ld((f == 0 ? sH : (f == 1 ? sU : sV)) + so);
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                r.a[e] = v.a[e] + ca * kk.a[e];
-                q.a[e] = (MODE == 1) ? cb * kk.a[e] : pa[LA ? f : 0].a[e] + cb * kk.a[e];
-            }
-            ov_st(Y1 + of, r);
-            ov_st(ACC + of, q);
-        } else {
-            V cm;
-            if constexpr (LC) cm = ov_ld(CMP + of);
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                const T inc = pa[LA ? f : 0].a[e] + (dt / T(6)) * kk.a[e];
-                if constexpr (sizeof(T) == 4) {
-                    r.a[e] = pv[LV ? f : 0].a[e];
-                    kahan_add(r.a[e], cm.a[e], inc);
-                } else {
-                    r.a[e] = pv[LV ? f : 0].a[e] + inc;
-                }
-            }
-            ov_st(V0 + of, r);
-            if constexpr (LC) ov_st(CMP + of, cm);
-        }
-    };
-    {
-        const V dx = one_x<1>(sJUT + so, ve, ec, we), ia = ov_ld(siJa + so),
-                dy = one_y<1, false, SW>(sJVT + SI(k, 0), (const T *)nullptr, j, n, xr);
-        V kk;
-#pragma unroll
-        for (int e = 0; e < VW; e++) kk.a[e] = (dx.a[e] * om.inv_hx + dy.a[e] * om.inv_hx) * ia.a[e];
+    // ---- P4: the tendencies of the tile's points and the RK4 update
+    if (touch) {
+        // the synchronised divergence of the boundary vertices; the gradient SAT across the edges;
+        // zeros in the elements beyond the fields' extent, which hold zeros and stay zero
+        const bool edgecol = k <= 1 || k + VW > n;
         if (j == 1 || j == n) {
 #pragma unroll
-            for (int e = 0; e < VW; e++) kk.a[e] = db[(j == 1 ? SIDE_B : SIDE_T) * L::HL + k + e - i0];
+            for (int e = 0; e < VW; e++) kh.a[e] = db[(j == 1 ? SIDE_B : SIDE_T) * L::HL + k + e - i0];
         }
-#pragma unroll
-        for (int e = 0; e < VW; e++) {
-            if (edgecol) {
-                if (k + e == 1) kk.a[e] = db[SIDE_L * L::HL + j - j0];
-                if (k + e == n) kk.a[e] = db[SIDE_R * L::HL + j - j0];
-                if (k + e > n) kk.a[e] = T(0);
-            }
-            kk.a[e] = -H * kk.a[e];
-        }
-        update(0, kk);
-    }
-    {
-        const T hx = ve < 0 ? T(0) : hh[(ve < HV ? SIDE_L : SIDE_R) * L::HL + j - j0];
-        const V gx = one_x<3>(sH + so, ve, ei, we, hx), cu = one_x<2>(sUP + so, ve, ei, we), ij = ov_ld(siJy + so);
-        V kk;
-#pragma unroll
-        for (int e = 0; e < VW; e++) {
-            kk.a[e] = -om.grav * (gx.a[e] * om.inv_hxa) + cu.a[e] * ij.a[e];
-            if (edgecol && k + e > N) kk.a[e] = T(0);
-        }
-        update(1, kk);
-    }
-    {
-        V kk = ov_zero<T, VW>();
-        if (j <= N) {
-            V gy = one_y<3, false, SW>(sH + SI(k, 0), (const T *)nullptr, j, N, xr);
-            const V cv = one_y<2, false, SW>(sVP + SI(k, 0), (const T *)nullptr, j, N, xr), ij = ov_ld(siJx + so);
-            if (j <= SB::NSAT || j >= N + 1 - SB::NSAT) {
-                const bool lo = j <= SB::NSAT;
-                const V hb = ov_ld(sH + SI(k, lo ? 1 : n));
-                const T *const ho = hh + (lo ? SIDE_B : SIDE_T) * L::HL + k - i0;
-                const T w = T(lo ? SB::satw(j) : -SB::satw(N + 1 - j));
-#pragma unroll
-                for (int e = 0; e < VW; e++) gy.a[e] += w * (hb.a[e] - ho[e]);
-            }
+        if (edgecol) {
 #pragma unroll
             for (int e = 0; e < VW; e++) {
-                kk.a[e] = -om.grav * (gy.a[e] * om.inv_hxa) + cv.a[e] * ij.a[e];
-                if (edgecol && k + e > n) kk.a[e] = T(0);
+                if (k + e == 1) kh.a[e] = db[SIDE_L * L::HL + j - j0];
+                if (k + e == n) kh.a[e] = db[SIDE_R * L::HL + j - j0];
+                if (k + e > n) kh.a[e] = T(0);
             }
         }
-        update(2, kk);
+        if (ve >= 0) {
+            const T hx = hh[(ve < HV ? SIDE_L : SIDE_R) * L::HL + j - j0];
+            const V w = ov_ld(we + ((3 * ONE_EDGES + ve) * ONE_TAPS + 8) * VW);
+#pragma unroll
+            for (int e = 0; e < VW; e++) ku.a[e] += w.a[e] * hx;
+        }
+        if (j <= SB::NSAT || (j >= N + 1 - SB::NSAT && j <= N)) {
+            const bool lo = j <= SB::NSAT;
+            const V hb = ov_ld(sH + SI(k, lo ? 1 : n));
+            const T *const ho = hh + (lo ? SIDE_B : SIDE_T) * L::HL + k - i0;
+            const T w = T(lo ? SB::satw(j) : -SB::satw(N + 1 - j));
+#pragma unroll
+            for (int e = 0; e < VW; e++) kv.a[e] += w * (hb.a[e] - ho[e]);
+        }
+    }
+    {
+        const V cu = one_x<2>(sUP + so, ve, ei, we), iy = ov_ld(siJy + so);
+#pragma unroll
+        for (int e = 0; e < VW; e++) {
+            kh.a[e] = -H * kh.a[e];
+            ku.a[e] = -om.grav * (ku.a[e] * om.inv_hxa) + cu.a[e] * iy.a[e];
+            if (k + e > N) ku.a[e] = T(0);
+        }
+        if (j <= N) {
+            const V cv = one_y<2, false, SW>(sVP + SI(k, 0), (const T *)nullptr, j, N, xr), ix = ov_ld(siJx + so);
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                kv.a[e] = -om.grav * (kv.a[e] * om.inv_hxa) + cv.a[e] * ix.a[e];
+                if (k + e > n) kv.a[e] = T(0);
+            }
+        }
+    }
+    if (mode == 0) {
+        ov_st(Y1 + po, kh);
+        ov_st(Y1 + po + fs, ku);
+        ov_st(Y1 + po + 2 * fs, kv);
+    } else if (mode <= 3) {
+        const T ca = (mode == 3) ? dt : T(0.5) * dt, cb = (mode == 1) ? dt / T(6) : dt / T(3);
+        if (mode == 1) {
+            pv[0] = ov_ld(sH + so);
+            pv[1] = ov_ld(sU + so);
+            pv[2] = ov_ld(sV + so);
+        }
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            const V &kk = f == 0 ? kh : (f == 1 ? ku : kv);
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                pv[f].a[e] = pv[f].a[e] + ca * kk.a[e];
+                pa[f].a[e] = pa[f].a[e] + cb * kk.a[e];   // (zero before, in mode 1)
+            }
+            ov_st(Y1 + po + f * fs, pv[f]);
+            ov_st(ACC + po + f * fs, pa[f]);
+        }
+    } else {
+        const T cb = dt / T(6);
+        V cm[3];
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int f = 0; f < 3; f++) cm[f] = ov_ld(CMP + po + f * fs);
+        }
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            const V &kk = f == 0 ? kh : (f == 1 ? ku : kv);
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                const T inc = pa[f].a[e] + cb * kk.a[e];
+                if constexpr (sizeof(T) == 4) kahan_add(pv[f].a[e], cm[f].a[e], inc);
+                else pv[f].a[e] = pv[f].a[e] + inc;
+            }
+            ov_st(V0 + po + f * fs, pv[f]);
+            if constexpr (sizeof(T) == 4) ov_st(CMP + po + f * fs, cm[f]);
+        }
     }
 }
 
