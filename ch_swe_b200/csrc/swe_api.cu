@@ -609,19 +609,25 @@ static int select_fused(swe_ctx *c, int th, int occ)
 // The one-launch stage's tables: the metric along the panel sides (from fmet, so the same
 // values) and the dense weights of the edge vectors.
 template <class T>
+struct OneTableSize {
+    static constexpr int NW = XROW_OPS * ONE_EDGES * ONE_TAPS * OV<T>::W, XR = NW, SIDE = (NW + XROW_LEN + 31) / 32 * 32;
+};
+template <class T>
 static int build_one_tables(swe_ctx *c)
 {
-    constexpr int VW = OV<T>::W, NW = XROW_OPS * ONE_EDGES * ONE_TAPS * VW;
-    const size_t ns = (size_t)4 * ONE_LINES * (c->cfg.N + 1), so = (NW + 31) / 32 * 32;
-    std::vector<double> w(NW);
-    one_edge_table(c->cfg.N, VW, w.data());
+    using Z = OneTableSize<T>;
+    const size_t ns = (size_t)4 * ONE_LINES * (c->cfg.N + 1);
+    std::vector<double> w(Z::NW + XROW_LEN);
+    one_edge_table(c->cfg.N, OV<T>::W, w.data());
+    xrow42_table(w.data() + Z::XR);
+    for (int q = 0; q < XROW_LEN; q++) w[Z::XR + q] *= (q / (XROW_ROWS * 5)) % 2 ? ONE_DS : ONE_IS;
     std::vector<T> wt(w.begin(), w.end());
     T *d = nullptr;
-    if (cudaMalloc(&d, (so + ns) * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "stage table allocation failed");
+    if (cudaMalloc(&d, (Z::SIDE + ns) * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "stage table allocation failed");
     c->onetab = d;
-    CU(c, cudaMemcpy(d, wt.data(), NW * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, cudaMemcpy(d, wt.data(), wt.size() * sizeof(T), cudaMemcpyHostToDevice));
     CU(c, cudaStreamSynchronize(cudaStreamLegacy));
-    OneTU<T>::tables((const T *)c->fmet, d + so, c->dims, c->stream);
+    OneTU<T>::tables((const T *)c->fmet, d + Z::SIDE, c->dims, c->stream);
     CU(c, cudaGetLastError());
     CU(c, cudaStreamSynchronize(c->stream));
     return SWE_OK;
@@ -629,9 +635,11 @@ static int build_one_tables(swe_ctx *c)
 template <class T>
 static OneMetric<T> one_metric(const swe_ctx *c, const MetricView<T> &mv)
 {
-    constexpr int NW = XROW_OPS * ONE_EDGES * ONE_TAPS * OV<T>::W;
+    using Z = OneTableSize<T>;
     const T *d = (const T *)c->onetab;
-    return OneMetric<T>{d + (NW + 31) / 32 * 32, d, mv.ea, mv.ef, mv.qb, mv.qt, mv.ql, mv.qr, mv.inv_hxa, mv.inv_hx, mv.grav};
+    const double hx = 0.5 * 3.141592653589793238462643383279502884 / c->cfg.N;
+    return OneMetric<T>{d + Z::SIDE, d, d + Z::XR, mv.ea, mv.ef, mv.qb, mv.qt, mv.ql, mv.qr, mv.inv_hx,
+                        T(1.0 / (ONE_DS * hx)), T(-c->cfg.grav / (ONE_DS * hx * c->cfg.radius))};
 }
 
 // Select the one-launch stage with configuration (label, occ).

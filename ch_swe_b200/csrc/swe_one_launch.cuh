@@ -24,13 +24,18 @@ enum { OS_JQ12 = 0, OS_JQN = 5, OS_IJN = 8, OS_JQT = 11, OS_IJT = 12 };
 // ninth, the neighbour's vertex value of the gradient SAT.
 constexpr int ONE_TAPS = 9, ONE_EDGES = 6;
 
+// Scales of the kernel's interpolations and differences (swe_onepass.cuh, one_row).
+constexpr double ONE_IS = -16.0, ONE_DS = -24.0;
+
 template <class T>
 struct OneMetric {
     const T *side;           // [4][ONE_LINES][n]
-    const T *we;             // [4 operators][ONE_EDGES][ONE_TAPS][VW]
+    const T *we;             // [4 operators][ONE_EDGES][ONE_TAPS][VW], scaled
+    const T *xr;             // xrow42_table's rows, scaled
     const T *ea, *ef;        // 1/(J a) and f J^2 of the boundary vertices (MetricView)
     const T *qb, *qt, *ql, *qr;
-    T inv_hxa, inv_hx, grav;
+    T inv_hx;
+    T cd, cg;                // 1 / (ONE_DS hx), -g / (ONE_DS hx a)
 };
 
 // The dense weights of the edge vectors of a cube of N cells (OneMetric::we), VW outputs per
@@ -65,6 +70,7 @@ static inline void one_edge_table(int N, int VW, double *we)
                 // the gradient SAT: satw (h(1) - halo) on the first rows, satw (halo - h(n)) on the last
                 if (op == 3 && k <= 3) { w[(1 - b) * VW] += satw[k - 1]; w[8 * VW] -= satw[k - 1]; }
                 if (op == 3 && k >= N - 2) { w[(n - b) * VW] -= satw[N - k]; w[8 * VW] += satw[N - k]; }
+                for (int m = 0; m < ONE_TAPS; m++) w[m * VW] *= (op & 1) ? ONE_DS : ONE_IS;
             }
         }
     }

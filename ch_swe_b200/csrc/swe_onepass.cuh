@@ -119,55 +119,94 @@ __device__ __forceinline__ void one_window(const T *p, T (&w)[OV<T>::W + 3])
     }
 }
 
+// Packed arithmetic: two FP32 operations per instruction on aligned register pairs
+// (fma.rn.f32x2), plain FP64.
+__device__ __forceinline__ uint64_t pk(float x, float y) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ void upk(uint64_t v, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+#define CHSWE_OV_OP(NAME, F32, F64)                                                                            \
+    __device__ __forceinline__ OV<float> NAME(const OV<float> &a, const OV<float> &b)                           \
+    {                                                                                                          \
+        OV<float> r;                                                                                           \
+        _Pragma("unroll") for (int e = 0; e < 4; e += 2) {                                                     \
+            uint64_t v;                                                                                        \
+            asm(F32 " %0, %1, %2;" : "=l"(v) : "l"(pk(a.a[e], a.a[e + 1])), "l"(pk(b.a[e], b.a[e + 1])));        \
+            upk(v, r.a[e], r.a[e + 1]);                                                                        \
+        }                                                                                                      \
+        return r;                                                                                              \
+    }                                                                                                          \
+    __device__ __forceinline__ OV<double> NAME(const OV<double> &a, const OV<double> &b)                        \
+    {                                                                                                          \
+        return OV<double>{{a.a[0] F64 b.a[0], a.a[1] F64 b.a[1]}};                                              \
+    }
+CHSWE_OV_OP(ov_add, "add.rn.f32x2", +)
+CHSWE_OV_OP(ov_sub, "sub.rn.f32x2", -)
+CHSWE_OV_OP(ov_mul, "mul.rn.f32x2", *)
+#undef CHSWE_OV_OP
+__device__ __forceinline__ OV<float> ov_fma(const OV<float> &a, const OV<float> &b, const OV<float> &c)
+{
+    OV<float> r;
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+        uint64_t v;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;"
+            : "=l"(v)
+            : "l"(pk(a.a[e], a.a[e + 1])), "l"(pk(b.a[e], b.a[e + 1])), "l"(pk(c.a[e], c.a[e + 1])));
+        upk(v, r.a[e], r.a[e + 1]);
+    }
+    return r;
+}
+__device__ __forceinline__ OV<double> ov_fma(const OV<double> &a, const OV<double> &b, const OV<double> &c)
+{
+    return OV<double>{{fma(a.a[0], b.a[0], c.a[0]), fma(a.a[1], b.a[1], c.a[1])}};
+}
 template <class T>
-__device__ __forceinline__ T one_mean(T v0, T v1, T v2, T v3) { return (T(9) * (v2 + v1) - (v3 + v0)) * T(0.0625); }
-template <class T>
-__device__ __forceinline__ T one_diff(T v0, T v1, T v2, T v3) { return (T(27) * (v2 - v1) - (v3 - v0)) * T(1.0 / 24.0); }
-template <bool D, class T>
-__device__ __forceinline__ OV<T> one_row4(const OV<T> &a, const OV<T> &b, const OV<T> &c, const OV<T> &d)
+__device__ __forceinline__ OV<T> ov_all(T x)
 {
     OV<T> r;
 #pragma unroll
-    for (int e = 0; e < OV<T>::W; e++)
-        r.a[e] = D ? one_diff(a.a[e], b.a[e], c.a[e], d.a[e]) : one_mean(a.a[e], b.a[e], c.a[e], d.a[e]);
+    for (int e = 0; e < OV<T>::W; e++) r.a[e] = x;
     return r;
 }
 
-// An edge vector: the dense weights of operator OP on the inputs row[0 .. 7] (and hx for
-// the difference of h).
+// Interior rows.  Every operator of this kernel is scaled, interpolations by -16 and
+// differences by -24: three operations per output, the scales folded into the constants
+// and metric products that follow (ONE_IS, ONE_DS; the closure weights carry them too).
+template <bool D, class T>
+__device__ __forceinline__ T one_row(T v0, T v1, T v2, T v3)
+{
+    return D ? fma(T(-27), v2 - v1, v3 - v0) : fma(T(-9), v2 + v1, v3 + v0);
+}
+template <bool D, class T>
+__device__ __forceinline__ OV<T> one_row4(const OV<T> &a, const OV<T> &b, const OV<T> &c, const OV<T> &d)
+{
+    if constexpr (D) return ov_fma(ov_all(T(-27)), ov_sub(c, b), ov_sub(d, a));
+    else return ov_fma(ov_all(T(-9)), ov_add(c, b), ov_add(d, a));
+}
+
+// An edge vector: the dense weights of operator OP on the inputs row[0 .. 7].
 template <int OP, class T>
-__device__ __forceinline__ OV<T> one_edge(const T *row, const T *we, T hx)
+__device__ __forceinline__ OV<T> one_edge(const T *row, const T *we)
 {
     constexpr int W = OV<T>::W;
-    OV<T> r = ov_zero<T, W>();
+    OV<T> r = ov_mul(*reinterpret_cast<const OV<T> *>(we), ov_all(row[0]));
 #pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const OV<T> w = *reinterpret_cast<const OV<T> *>(we + m * W);
-        const T x = row[m];
-#pragma unroll
-        for (int e = 0; e < W; e++) r.a[e] += w.a[e] * x;
-    }
-    if constexpr (OP == 3) {
-        const OV<T> w = *reinterpret_cast<const OV<T> *>(we + 8 * W);
-#pragma unroll
-        for (int e = 0; e < W; e++) r.a[e] += w.a[e] * hx;
-    }
+    for (int m = 1; m < 8; m++) r = ov_fma(*reinterpret_cast<const OV<T> *>(we + m * W), ov_all(row[m]), r);
     return r;
 }
 
 // Operator OP (0 I_c2i, 1 D_c2i, 2 I_i2c, 3 D_i2c) along x on the VW outputs at p; ve >= 0:
 // an edge vector, whose inputs start eo points from p.
 template <int OP, class T>
-__device__ __forceinline__ OV<T> one_x(const T *p, int ve, int eo, const T *we, T hx = T(0))
+__device__ __forceinline__ OV<T> one_x(const T *p, int ve, int eo, const T *we)
 {
     constexpr int W = OV<T>::W;
-    if (ve >= 0) return one_edge<OP, T>(p + eo, we + (OP * ONE_EDGES + ve) * ONE_TAPS * W, hx);
+    if (ve >= 0) return one_edge<OP, T>(p + eo, we + (OP * ONE_EDGES + ve) * ONE_TAPS * W);
     T w[W + 3];
     one_window<(OP <= 1 ? -2 : -1)>(p, w);
     OV<T> r;
 #pragma unroll
     for (int e = 0; e < W; e++)
-        r.a[e] = (OP & 1) ? one_diff(w[e], w[e + 1], w[e + 2], w[e + 3]) : one_mean(w[e], w[e + 1], w[e + 2], w[e + 3]);
+        r.a[e] = one_row<(OP & 1) != 0>(w[e], w[e + 1], w[e + 2], w[e + 3]);
     return r;
 }
 
@@ -175,14 +214,6 @@ template <class T>
 __device__ __forceinline__ OV<T> ov_ld(const T *p) { return *reinterpret_cast<const OV<T> *>(p); }
 template <class T>
 __device__ __forceinline__ void ov_st(T *p, const OV<T> &v) { *reinterpret_cast<OV<T> *>(p) = v; }
-template <class T>
-__device__ __forceinline__ OV<T> ov_mul(const OV<T> &a, const OV<T> &b)
-{
-    OV<T> r;
-#pragma unroll
-    for (int e = 0; e < OV<T>::W; e++) r.a[e] = a.a[e] * b.a[e];
-    return r;
-}
 
 // The weight row of operator op (xrow42's rows) at output k of nm: first input and the table's row.
 __device__ __forceinline__ void one_rowsel(int op, int k, int nm, int &base, int &w)
@@ -212,14 +243,9 @@ __device__ __forceinline__ OV<T> one_y(const T *col, const T *col2, int l, int n
     }
     int base, w;
     one_rowsel(OP, l, nm, base, w);
-    OV<T> r = ov_zero<T, OV<T>::W>();
+    OV<T> r = ov_mul(ov_all(xr[w]), at(base));
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const T c = xr[w + m];
-        const OV<T> v = at(base + m);
-#pragma unroll
-        for (int e = 0; e < OV<T>::W; e++) r.a[e] += c * v.a[e];
-    }
+    for (int m = 1; m < 5; m++) r = ov_fma(ov_all(xr[w + m]), at(base + m), r);
     return r;
 }
 
@@ -344,8 +370,8 @@ __global__ void __maxnreg__(REGS)
         for (int m = 0; m < 5; m++) wI[m] = wD[m] = wC[m] = T(0);
         const T *const gx = xrow_table<T>();
         if (node) {
-            fo = __ldg(om.ef + (t * 4 + s) * n + al - 1);
-            fn = __ldg(om.ef + (K.nb * 4 + K.nside) * n + y - 1);
+            fo = T(ONE_IS) * __ldg(om.ef + (t * 4 + s) * n + al - 1);
+            fn = T(ONE_IS) * __ldg(om.ef + (K.nb * 4 + K.nside) * n + y - 1);
             eao = __ldg(om.ea + s * n + al - 1);
             ean = __ldg(om.ea + K.nside * n + y - 1);
             qs = __ldg((s == SIDE_L ? om.ql : (s == SIDE_R ? om.qr : (s == SIDE_B ? om.qb : om.qt))) + al - 1);
@@ -539,19 +565,21 @@ __global__ void __maxnreg__(REGS)
         else if (v >= vr && v < NV) { ve = HV + (v - vr); ec = N - 7 - k; ei = n - 7 - k; }
     }
     if (touch) {
-        const T *const gx = xrow_table<T>();
-        for (int q = tid; q < XROW_LEN; q += NM) xr[q] = __ldg(gx + q);
-        for (int q = tid; q < XROW_OPS * ONE_EDGES * ONE_TAPS; q += NM)
+        for (int q = tid; q < XROW_LEN; q += NM) xr[q] = __ldg(om.xr + q);
+        for (int q = tid; q < XROW_OPS * ONE_EDGES * ONE_TAPS && (touch & 3u); q += NM)
             ov_st(we + q * VW, *reinterpret_cast<const V *>(om.we + q * VW));
     }
     const T H = T(__ldg(a.Hm + mem)), dt = T(a.dtm ? __ldg(a.dtm + mem) : a.dt);
-    nbar_sync(BAR_MAIN, NM);                              // the barrier's initialisation, the tables
-    if (!mbar_wait(bar, 0, FUSED_WAIT_NS)) {
+    // the first warp waits for the tile loads (its first thread initialised the barrier), the others
+    // at the named barrier, where they take no issue slots
+    __syncwarp();
+    if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
         // the tile loads did not arrive: record it, wait once more (bounded), and finish on
         // whatever the windows hold
         atomicExch(err, 1);
         mbar_wait(bar, 0, FUSED_WAIT_NS);
     }
+    nbar_sync(BAR_MAIN, NM);
     pdl_wait();                                           // (the loads waited already)
 
     // ---- P1: vq = JQ12 I_c2i,y(v) on rows [j0-1, j1+2), uq = JQ12 I_c2i,x(u) on rows [j0-3, j1+3)
@@ -572,27 +600,20 @@ __global__ void __maxnreg__(REGS)
     // ---- P2: J ut = JQ11 u + I_i2c,x(vq) on u points, rows [j0-1, j1+2); ut = J ut / J
     //          J vt = JQ22 v + I_i2c,y(uq) on v points, rows [j0-2, j1+1)
     {
+        const V s2 = ov_all(T(1.0 / (ONE_IS * ONE_IS)));
         const int l = max(j0 - 1, 1) + ty;
         if (lane_ok && l < min(j1 + 2, n + 1)) {
             const int o = SI(k, l);
-            const V I = one_x<2>(sVQ + o, ve, ei, we), u = ov_ld(sU + o), q = ov_ld(sJQ11 + o), ij = ov_ld(siJy + o);
-            V r, w;
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                r.a[e] = q.a[e] * u.a[e] + I.a[e];
-                w.a[e] = r.a[e] * ij.a[e];
-            }
+            const V I = one_x<2>(sVQ + o, ve, ei, we);
+            const V r = ov_fma(I, s2, ov_mul(ov_ld(sJQ11 + o), ov_ld(sU + o)));
             ov_st(sJUT + o, r);
-            ov_st(sUT + o, w);
+            ov_st(sUT + o, ov_mul(r, ov_ld(siJy + o)));
         }
         const int m = max(j0 - 2, 1) + ty;
         if (lane_ok && m < min(j1 + 1, N + 1)) {
             const int o = SI(k, m);
-            const V I = one_y<2, false, SW>(sUQ + SI(k, 0), (const T *)nullptr, m, N, xr), v = ov_ld(sV + o), q = ov_ld(sJQ22 + o);
-            V r;
-#pragma unroll
-            for (int e = 0; e < VW; e++) r.a[e] = q.a[e] * v.a[e] + I.a[e];
-            ov_st(sJVT + o, r);
+            const V I = one_y<2, false, SW>(sUQ + SI(k, 0), (const T *)nullptr, m, N, xr);
+            ov_st(sJVT + o, ov_fma(I, s2, ov_mul(ov_ld(sJQ22 + o), ov_ld(sV + o))));
         }
     }
     nbar_sync(BAR_MAIN, NM);
@@ -646,12 +667,10 @@ __global__ void __maxnreg__(REGS)
         }
         // the parts that need no boundary value: divergence and gradient (without the SAT's
         // neighbour terms)
-        {
-            const V dx = one_x<1>(sJUT + so, ve, ec, we), ia = ov_ld(siJa + so),
-                    dy = one_y<1, false, SW>(sJVT + SI(k, 0), (const T *)nullptr, j, n, xr);
-#pragma unroll
-            for (int e = 0; e < VW; e++) kh.a[e] = (dx.a[e] * om.inv_hx + dy.a[e] * om.inv_hx) * ia.a[e];
-        }
+        kh = ov_mul(ov_mul(ov_add(one_x<1>(sJUT + so, ve, ec, we),
+                                  one_y<1, false, SW>(sJVT + SI(k, 0), (const T *)nullptr, j, n, xr)),
+                           ov_all(om.cd)),
+                    ov_ld(siJa + so));
         ku = one_x<3>(sH + so, ve, ei, we);
         kv = ov_zero<T, VW>();
         if (j <= N) kv = one_y<3, false, SW>(sH + SI(k, 0), (const T *)nullptr, j, N, xr);
@@ -662,8 +681,7 @@ __global__ void __maxnreg__(REGS)
 
     // ---- P4: the tendencies of the tile's points and the RK4 update
     if (touch) {
-        // the synchronised divergence of the boundary vertices; the gradient SAT across the edges;
-        // zeros in the elements beyond the fields' extent, which hold zeros and stay zero
+        // the synchronised divergence of the boundary vertices; the gradient SAT across the edges
         const bool edgecol = k <= 1 || k + VW > n;
         if (j == 1 || j == n) {
 #pragma unroll
@@ -674,41 +692,36 @@ __global__ void __maxnreg__(REGS)
             for (int e = 0; e < VW; e++) {
                 if (k + e == 1) kh.a[e] = db[SIDE_L * L::HL + j - j0];
                 if (k + e == n) kh.a[e] = db[SIDE_R * L::HL + j - j0];
-                if (k + e > n) kh.a[e] = T(0);
             }
         }
         if (ve >= 0) {
             const T hx = hh[(ve < HV ? SIDE_L : SIDE_R) * L::HL + j - j0];
-            const V w = ov_ld(we + ((3 * ONE_EDGES + ve) * ONE_TAPS + 8) * VW);
-#pragma unroll
-            for (int e = 0; e < VW; e++) ku.a[e] += w.a[e] * hx;
+            ku = ov_fma(ov_ld(we + ((3 * ONE_EDGES + ve) * ONE_TAPS + 8) * VW), ov_all(hx), ku);
         }
         if (j <= SB::NSAT || (j >= N + 1 - SB::NSAT && j <= N)) {
             const bool lo = j <= SB::NSAT;
             const V hb = ov_ld(sH + SI(k, lo ? 1 : n));
             const T *const ho = hh + (lo ? SIDE_B : SIDE_T) * L::HL + k - i0;
-            const T w = T(lo ? SB::satw(j) : -SB::satw(N + 1 - j));
+            const T w = T(ONE_DS * (lo ? SB::satw(j) : -SB::satw(N + 1 - j)));
 #pragma unroll
             for (int e = 0; e < VW; e++) kv.a[e] += w * (hb.a[e] - ho[e]);
         }
     }
     {
-        const V cu = one_x<2>(sUP + so, ve, ei, we), iy = ov_ld(siJy + so);
-#pragma unroll
-        for (int e = 0; e < VW; e++) {
-            kh.a[e] = -H * kh.a[e];
-            ku.a[e] = -om.grav * (ku.a[e] * om.inv_hxa) + cu.a[e] * iy.a[e];
-            if (k + e > N) ku.a[e] = T(0);
-        }
-        if (j <= N) {
-            const V cv = one_y<2, false, SW>(sVP + SI(k, 0), (const T *)nullptr, j, N, xr), ix = ov_ld(siJx + so);
+        const V s2 = ov_all(T(1.0 / (ONE_IS * ONE_IS))), cg = ov_all(om.cg);
+        kh = ov_mul(kh, ov_all(-H));
+        ku = ov_fma(ov_mul(one_x<2>(sUP + so, ve, ei, we), ov_ld(siJy + so)), s2, ov_mul(ku, cg));
+        if (j <= N)
+            kv = ov_fma(ov_mul(one_y<2, false, SW>(sVP + SI(k, 0), (const T *)nullptr, j, N, xr), ov_ld(siJx + so)), s2,
+                        ov_mul(kv, cg));
+        if (k + VW > n)
 #pragma unroll
             for (int e = 0; e < VW; e++) {
-                kv.a[e] = -om.grav * (kv.a[e] * om.inv_hxa) + cv.a[e] * ix.a[e];
-                if (k + e > n) kv.a[e] = T(0);
+                if (k + e > N) ku.a[e] = T(0);
+                if (k + e > n) kh.a[e] = kv.a[e] = T(0);
             }
-        }
     }
+    // elements beyond the fields' extent hold zeros and stay zero
     if (mode == 0) {
         ov_st(Y1 + po, kh);
         ov_st(Y1 + po + fs, ku);
@@ -723,11 +736,8 @@ __global__ void __maxnreg__(REGS)
 #pragma unroll
         for (int f = 0; f < 3; f++) {
             const V &kk = f == 0 ? kh : (f == 1 ? ku : kv);
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                pv[f].a[e] = pv[f].a[e] + ca * kk.a[e];
-                pa[f].a[e] = pa[f].a[e] + cb * kk.a[e];   // (zero before, in mode 1)
-            }
+            pv[f] = ov_fma(ov_all(ca), kk, pv[f]);
+            pa[f] = ov_fma(ov_all(cb), kk, pa[f]);   // (zero before, in mode 1)
             ov_st(Y1 + po + f * fs, pv[f]);
             ov_st(ACC + po + f * fs, pa[f]);
         }
