@@ -24,16 +24,21 @@ FUSED_SOURCES = ["fused_f.cu", "fused_d.cu"]
 GROUP_SOURCES = ["group_f.cu", "group_d.cu"]
 # the one-launch linear stage, one unit per precision
 ONE_SOURCES = ["one_f.cu", "one_d.cu"]
-SOURCES = ["swe_api.cu", *STAGE_SOURCES, *FUSED_SOURCES, *GROUP_SOURCES, *ONE_SOURCES]
+# the advective operator's vector kernels, one unit per precision
+ADVONE_SOURCES = ["advone_f.cu", "advone_d.cu"]
+SOURCES = ["swe_api.cu", *STAGE_SOURCES, *FUSED_SOURCES, *GROUP_SOURCES, *ONE_SOURCES, *ADVONE_SOURCES]
 COMMON_HEADERS = ["swe_common.cuh", "swe_kernels.cuh", "swe_sbp.cuh", "sbp63.h", "swe_advective.cuh", "swe_launch.cuh",
                   "swe_fused.cuh", "swe_tma.cuh"]
-UNIT_HEADERS = {"swe_api.cu": COMMON_HEADERS + ["swe_ah.cuh", "swe_cgrid.cuh", "swe_diff.cuh", "lap63.h", "swe_one_launch.cuh"],
+UNIT_HEADERS = {"swe_api.cu": COMMON_HEADERS + ["swe_ah.cuh", "swe_cgrid.cuh", "swe_diff.cuh", "lap63.h", "swe_one_launch.cuh",
+                                                "swe_adv_launch.cuh"],
                 **{src: COMMON_HEADERS + ["fused_tu.cuh"] for src in FUSED_SOURCES},
-                **{src: COMMON_HEADERS + ["swe_onepass.cuh", "swe_one_launch.cuh", "one_tu.cuh"] for src in ONE_SOURCES}}
+                **{src: COMMON_HEADERS + ["swe_onepass.cuh", "swe_one_launch.cuh", "one_tu.cuh"] for src in ONE_SOURCES},
+                **{src: COMMON_HEADERS + ["swe_onepass.cuh", "swe_one_launch.cuh", "one_tu.cuh", "swe_adv_launch.cuh",
+                                          "swe_advone.cuh", "advone_tu.cuh"] for src in ADVONE_SOURCES}}
 STAGE_HEADERS = COMMON_HEADERS + ["swe_tiled.cuh", "swe_stage_tu.cuh"]
 UNIT_HEADERS.update({src: COMMON_HEADERS + ["swe_tiled.cuh", "swe_group.cuh", "group_tu.cuh"] for src in GROUP_SOURCES})
 HEADERS = sorted(set(COMMON_HEADERS + UNIT_HEADERS["swe_api.cu"] + STAGE_HEADERS + ["fused_tu.cuh", "swe_group.cuh", "group_tu.cuh",
-                                                                                    "one_tu.cuh", "swe_onepass.cuh"]))
+                                                                                    "one_tu.cuh", "swe_onepass.cuh", "swe_advone.cuh", "advone_tu.cuh"]))
 DEPS = SOURCES + HEADERS
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

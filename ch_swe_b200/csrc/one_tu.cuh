@@ -84,8 +84,9 @@ void OneTU<T>::tables(const T *fmet, T *side, const Dims &d, cudaStream_t st)
     k_one_tables<T><<<dim3((d.N + 1 + 127) / 128, 4), 128, 0, st>>>(fmet, side, d);
 }
 
+// This translation unit's copies of the panel links and the closure rows.
 template <class T>
-cudaError_t OneTU<T>::upload_tables(const Link *links)
+static cudaError_t one_upload(const Link *links)
 {
     cudaError_t e = cudaMemcpyToSymbol(c_link, links, sizeof(Link) * NPAN * 4);
     double w[XROW_LEN];
@@ -97,6 +98,12 @@ cudaError_t OneTU<T>::upload_tables(const Link *links)
         else e = cudaMemcpyToSymbol(g_xrow_d, wt, sizeof(wt));
     }
     return e;
+}
+
+template <class T>
+cudaError_t OneTU<T>::upload_tables(const Link *links)
+{
+    return one_upload<T>(links);
 }
 
 }  // namespace chswe

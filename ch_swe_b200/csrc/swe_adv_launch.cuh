@@ -1,0 +1,29 @@
+// swe_adv_launch.cuh -- host-side entry points of the advective operator's vector kernels
+// (swe_advone.cuh) of one precision.
+#pragma once
+
+#include "swe_advective.cuh"
+#include "swe_one_launch.cuh"
+
+namespace chswe {
+
+// Configurations of k_adv_stage and k_adv_co2: (label, XL, TH, blocks per SM, registers).
+#define CHSWE_ADVONE_CFGS_F(X) X(25, 10, 21, 2, 64) X(33, 10, 29, 2, 64)
+#define CHSWE_ADVONE_CFGS_D(X) X(17, 16, 15, 2, 64) X(25, 16, 23, 1, 96)
+
+template <class T>
+struct AdvOneTU {
+    static cudaError_t optin();
+    static bool box(int label, int occ, int &w, int &h);
+    static bool grid(int label, int occ, int N, int members, OneGrid &g);
+    static bool co2(int label, int occ, int members, const CUtensorMap &tmY, T *w, const Dims &d, const OneMetric<T> &om,
+                    const T *fmet, const double *dtm, int *err, cudaStream_t st);
+    static void flux(int members, const T *y, const T *w, T *f, const Dims &d, const AdvView<T> &av, const MetricView<T> &m,
+                     const double *dtm, cudaStream_t st);
+    static bool stage(int label, int occ, int members, const CUtensorMap &tmY, const CUtensorMap &tmW, const CUtensorMap &tmF,
+                      const CUtensorMap &tmM, const T *w, T *v0, T *y1, T *acc, T *cmp, const Dims &d, const OneMetric<T> &om,
+                      const StageArgs &a, int *err, cudaStream_t st);
+    static cudaError_t upload_tables(const Link *links);
+};
+
+}  // namespace chswe

@@ -22,6 +22,7 @@
 #include "swe_kernels.cuh"
 #include "swe_launch.cuh"
 #include "swe_one_launch.cuh"
+#include "swe_adv_launch.cuh"
 
 namespace chswe {
 
@@ -407,6 +408,8 @@ static cudaError_t upload_link_tables()
     if (e == cudaSuccess) e = FusedTU<double>::upload_tables(l);
     if (e == cudaSuccess) e = OneTU<float>::upload_tables(l);
     if (e == cudaSuccess) e = OneTU<double>::upload_tables(l);
+    if (e == cudaSuccess) e = AdvOneTU<float>::upload_tables(l);
+    if (e == cudaSuccess) e = AdvOneTU<double>::upload_tables(l);
     if (e == cudaSuccess) e = GroupTU<float>::upload_tables(l, q);
     if (e == cudaSuccess) e = GroupTU<double>::upload_tables(l, q);
     return e;
@@ -642,15 +645,23 @@ static OneMetric<T> one_metric(const swe_ctx *c, const MetricView<T> &mv)
                         T(1.0 / (ONE_DS * hx)), T(-c->cfg.grav / (ONE_DS * hx * c->cfg.radius))};
 }
 
-// Select the one-launch stage with configuration (label, occ).
-static int select_one(swe_ctx *c, int label, int occ)
+// The vector stage's TMA boxes of configuration (label, occ): the one-launch stage, or the
+// advective operator's; false: not built, or the cube's tiles do not suit it.
+template <class T>
+static bool one_box(const swe_ctx *c, int label, int occ, int &bw, int &bh)
 {
     OneGrid og;
+    const int N = c->cfg.N, M = c->cfg.n_members;
+    if (c->adv) return AdvOneTU<T>::box(label, occ, bw, bh) && AdvOneTU<T>::grid(label, occ, N, M, og);
+    return OneTU<T>::box(label, occ, bw, bh) && OneTU<T>::grid(label, occ, N, M, og);
+}
+
+// Select the one-launch stage (the advective operator's vector stage) with configuration (label, occ).
+static int select_one(swe_ctx *c, int label, int occ)
+{
     int bw = 0, bh = 0;
     const bool f64 = c->elem == 8;
-    const bool built = f64 ? OneTU<double>::box(label, occ, bw, bh) && OneTU<double>::grid(label, occ, c->cfg.N, c->cfg.n_members, og)
-                           : OneTU<float>::box(label, occ, bw, bh) && OneTU<float>::grid(label, occ, c->cfg.N, c->cfg.n_members, og);
-    if (!fused_supported(c) || c->cstag || !built)
+    if (c->ah || c->cstag || c->ord != 42 || !(f64 ? one_box<double>(c, label, occ, bw, bh) : one_box<float>(c, label, occ, bw, bh)))
         return fail(c, SWE_EINVAL, "one-launch stage configuration (%d, %d) is not available for this context", label, occ);
     if (int rc = ensure_fused_metric(c)) return rc;
     if (!c->onetab)
@@ -1097,11 +1108,15 @@ static cudaError_t stage_smem_optin();
 // against 102 us) and small cubes with many members are faster split (64 x C48: 496 against
 // 425 us: every tile holds a panel corner).
 template <class T>
-static KernelCfg one_default_cfg(int N, int members)
+static KernelCfg one_default_cfg(int N, int members, bool adv)
 {
     OneGrid og;
     const KernelCfg none{0, 0, 0};
     if (N < 16) return none;
+    if (adv) {
+        const KernelCfg k = sizeof(T) == 4 ? KernelCfg{33, 2, 3} : KernelCfg{17, 2, 3};
+        return AdvOneTU<T>::grid(k.tile, k.occ, N, members, og) ? k : none;
+    }
     if (sizeof(T) == 4) return OneTU<T>::grid(33, 2, N, members, og) ? KernelCfg{33, 2, 3} : none;
     if (N < 128 && members > 4) return none;
     for (int label : {25, 33})
@@ -1205,8 +1220,8 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
             }
         }
     }
-    if (fused_supported(c) && !c->cstag) {
-        const KernelCfg k = c->elem == 8 ? one_default_cfg<double>(N, cfg->n_members) : one_default_cfg<float>(N, cfg->n_members);
+    if (!c->ah && !c->cstag && ord == 42) {
+        const KernelCfg k = c->elem == 8 ? one_default_cfg<double>(N, cfg->n_members, c->adv) : one_default_cfg<float>(N, cfg->n_members, c->adv);
         if (k.tile) {
             if ((rc = select_one(c, k.tile, k.occ)) != SWE_OK) return bail(rc);
             c->one_default = true;
@@ -1524,6 +1539,7 @@ static cudaError_t stage_smem_optin()
     if (e == cudaSuccess) e = StageTU<T, 33>::optin();
     if (e == cudaSuccess) e = FusedTU<T>::optin();
     if (e == cudaSuccess) e = OneTU<T>::optin();
+    if (e == cudaSuccess) e = AdvOneTU<T>::optin();
     if (e == cudaSuccess) e = GroupTU<T>::optin();
     if (e == cudaSuccess) e = set_carveout(k_edge<T, 42>);
     if (e == cudaSuccess) e = set_carveout(k_edge<T, 21>);
@@ -1649,6 +1665,57 @@ static void launch_adv(swe_ctx *c, const void *yin, const AdvView<T> &av, const 
                  (const T *)c->w, (const T *)c->vh, (T *)c->adt, c->dims, av, mv, dtm);
 }
 
+// One stage of the advective operator through its vector kernels (swe_advone.cuh), six
+// launches; false: a tensor map cannot be encoded and nothing was launched.
+template <class T>
+static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, void *acc, float *cmp, int mode, double dt,
+                            const double *dtm, const MetricView<T> &mv, bool fork)
+{
+    const int M = c->cfg.n_members, N = c->cfg.N;
+    const AdvView<T> &av = adv_view<T>(c);
+    const int64_t nrows = (int64_t)M * 3 * NPAN * (N + 1 + 2 * MG);
+    int bw, bh;
+    CUtensorMap tmY, tmW, tmF;
+    if (!one_box<T>(c, c->olabel, c->oocc, bw, bh) || !encode_rows(&tmY, yin, sizeof(T), c->dims.P, nrows, bw, bh) ||
+        !encode_rows(&tmW, c->w, sizeof(T), c->dims.P, nrows, bw, bh) || !encode_rows(&tmF, c->fl, sizeof(T), c->dims.P, nrows, bw, bh))
+        return false;
+    const OneMetric<T> om = one_metric<T>(c, mv);
+    const dim3 hg(1 + (12 * (N - 1) + HAVG_THREADS - 1) / HAVG_THREADS, M);
+    const dim3 vg((unsigned)(((long long)NPAN * av.hp * M + 255) / 256));
+    cudaStream_t st = c->stream, sd = fork ? c->side : c->stream;
+    auto co2 = [&] { AdvOneTU<T>::co2(c->olabel, c->oocc, M, tmY, (T *)c->w, c->dims, om, (const T *)c->fmet, dtm, c->derr, st); };
+    auto havg = [&] { launch_k(k_havg<T>, hg, dim3(HAVG_THREADS), 0, sd, (T *)yin, (T *)c->hb, c->dims, dtm); };
+    auto vhalo = [&] { launch_k(k_vhalo<T>, vg, dim3(256), 0, sd, (const T *)yin, (T *)c->vh, c->dims, av, M, dtm); };
+    auto flux = [&] { AdvOneTU<T>::flux(M, (const T *)yin, (const T *)c->w, (T *)c->fl, c->dims, av, mv, dtm, st); };
+    if (fork) {
+        // the averaging of h, the wind halo and the advective tendencies beside co2 and the flux
+        cudaEventRecord(c->ev_fork, st);
+        cudaStreamWaitEvent(sd, c->ev_fork, 0);
+        havg();
+        cudaEventRecord(c->ev_havg, sd);
+        vhalo();
+        co2();
+        cudaEventRecord(c->ev_co2, st);
+        cudaStreamWaitEvent(sd, c->ev_co2, 0);
+        launch_adv<T>(c, yin, av, mv, dtm, sd);
+        cudaEventRecord(c->ev_side, sd);
+        cudaStreamWaitEvent(st, c->ev_havg, 0);
+        flux();
+        cudaStreamWaitEvent(st, c->ev_side, 0);
+    } else {
+        co2();
+        havg();
+        vhalo();
+        launch_adv<T>(c, yin, av, mv, dtm, st);
+        flux();
+    }
+    StageArgs a{mode, dt, c->ones, dtm, c->fl, c->adt, c->hb, c->hs};
+    AdvOneTU<T>::stage(c->olabel, c->oocc, M, tmY, tmW, tmF, c->tm_one, (const T *)c->w, (T *)v0, (T *)y1, (T *)acc, (T *)cmp,
+                       c->dims, om, a, c->derr, st);
+    c->launches += 6;
+    return true;
+}
+
 template <class T>
 static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void *acc, float *cmp, int mode, double dt,
                           const double *dtm,
@@ -1697,6 +1764,11 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
     const long long nvh = (long long)NPAN * av.hp * M;
     const dim3 vg((unsigned)((nvh + 255) / 256));
     const bool fork = c->side && c->branches;
+    if (c->one) {
+        if (enqueue_adv_one<T>(c, yin, v0, y1, acc, cmp, mode, dt, dtm, mv, fork)) return;
+        c->one = false;
+        c->err = "vector stage unavailable (TMA tensor map); using the split stage kernels";
+    }
     if (fork) {
         // The averaging of h and the wind halo depend on the stage input only, the
         // wind at the vertices and the advective tendencies (which read neither h
@@ -3936,9 +4008,18 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
         }
 #undef CHSWE_OADD
     }
+    if (c->adv && c->ord == 42) {
+#define CHSWE_OADD(LABEL, XL, TH, OCC, REGS) all.push_back(KernelCfg{LABEL, OCC, 3});
+        if (c->elem == 4) {
+            CHSWE_ADVONE_CFGS_F(CHSWE_OADD)
+        } else {
+            CHSWE_ADVONE_CFGS_D(CHSWE_OADD)
+        }
+#undef CHSWE_OADD
+    }
     for (size_t k = 0; k < all.size() && rc == SWE_OK; k++) {
         const KernelCfg kc = all[k];
-        if (c->adv && kc.occ != default_occ(kc.tile)) continue;
+        if (c->adv && kc.runs < 2 && kc.occ != default_occ(kc.tile)) continue;
         if (apply_cfg(c, kc.tile, kc.occ, kc.runs) != SWE_OK) continue;   // a fused tile the cube cannot take
         // untimed: capture and instantiate the graphs the timed steps replay
         if ((rc = swe_rk4_steps(c, v, dt, warm)) != SWE_OK) break;

@@ -111,3 +111,41 @@ def test_default_stage_matches_oracle_and_joins_a_group():
         assert rel(a, r) < 1e-12
     g.destroy()
     dom.destroy()
+
+
+ADV_CFGS = [("fp64", c) for c in ((17, 2, 3), (25, 1, 3))] + [("fp32", c) for c in ((25, 2, 3), (33, 2, 3))]
+
+
+@pytest.mark.parametrize("orography", [False, True])
+@pytest.mark.parametrize("precision,cfg", ADV_CFGS)
+@pytest.mark.parametrize("N", [16, 23, 24, 31, 33, 34, 46, 65, 79])
+def test_advective_apply_matches_oracle(precision, cfg, N, orography):
+    """The advective operator's vector kernels: random winds and disagreeing edge copies on a
+    full depth, with and without orography."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator
+    from oracle.oracle import Oracle
+    rng = np.random.default_rng(70 + N)
+    h, u, v = random_state(N, 300 + N)
+    h = 1000.0 + 50.0 * h
+    hs = 100.0 * rng.standard_normal(h.shape) if orography else None
+    axis = (0.3, -0.5, 0.8)
+    o = Oracle(N, axis=axis, operator="advective")
+    if orography:
+        o.set_orography(hs)
+    ref = o.apply(h, u, v)
+    dom = create_domain(N, precision=precision, rotation_axis=axis, operator="advective")
+    try:
+        dom.kernel_config = cfg
+    except SweError:
+        assert cfg[1] == 1 and N <= 24
+        return
+    assert dom.kernel_config == cfg
+    op = create_swm_operator(dom.grav, {"swm_operator_type": "advective_swm_operator"}, dom)
+    if orography:
+        op.set_orography(hs)
+    x, y = create_stvec_swm(dom).upload(h, u, v), create_stvec_swm(dom)
+    op.apply(y, x, dom)
+    dom.synchronize()
+    for g, r, name in zip(y.download(), ref, "huv"):
+        assert rel(g, r) < RTOL[precision], (name, rel(g, r))
+    dom.destroy()
