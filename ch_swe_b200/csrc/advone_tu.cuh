@@ -22,6 +22,10 @@ static cudaError_t advone_optin()
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_adv_co2<T, XL, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)CoLayout<T, XL, TH>::bytes());
+    if constexpr (sizeof(T) == 4)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_adv_tend<T, XL, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TendLayout<T, XL, TH>::bytes());
     return e;
 }
 
@@ -80,11 +84,31 @@ bool AdvOneTU<T>::co2(int label, int occ, int members, const CUtensorMap &tmY, T
 }
 
 template <class T>
+bool AdvOneTU<T>::tend(int label, int occ, int members, const CUtensorMap &tmY, const CUtensorMap &tmW, const T *vh, T *adt,
+                       const Dims &d, const AdvView<T> &av, const OneMetric<T> &om, T inv_hxa, const double *dtm, int *err,
+                       cudaStream_t st)
+{
+    OneGrid og;
+    if (sizeof(T) == 8 || !grid(label, occ, d.N, members, og)) return false;
+#define CHSWE_O(LABEL, XL, TH, OCC, REGS)                                                                               \
+    if (label == LABEL && occ == OCC) {                                                                                 \
+        if constexpr (sizeof(T) == 4)                                                                                   \
+        launch_k(k_adv_tend<T, XL, TH>, og.g, dim3(TendLayout<T, XL, TH>::NM), TendLayout<T, XL, TH>::bytes(), st, tmY, \
+                 tmW, vh, adt, d, av, om, inv_hxa, og.t, dtm, err);                                                     \
+        return true;                                                                                                    \
+    }
+    CHSWE_ADVONE_EACH(CHSWE_O)
+#undef CHSWE_O
+    return false;
+}
+
+template <class T>
 void AdvOneTU<T>::flux(int members, const T *y, const T *w, T *f, const Dims &d, const AdvView<T> &av, const MetricView<T> &m,
                        const double *dtm, cudaStream_t st)
 {
-    const int n = d.N + 1, nv = (n + OV<T>::W - 1) / OV<T>::W;
-    launch_k(k_adv_flux<T>, dim3((nv + 31) / 32, (n + 7) / 8, NPAN * members), dim3(32, 8), 0, st, y, w, f, d, av, m, dtm);
+    const int n = d.N + 1, nv = (n + OV<T>::W - 1) / OV<T>::W, gx = (nv + 31) / 32, ny = (n + 7) / 8;
+    const int ne = (flux_edge_items(d.N, OV<T>::W) + 256 * gx - 1) / (256 * gx);
+    launch_k(k_adv_flux<T>, dim3(gx, ny + ne, NPAN * members), dim3(32, 8), 0, st, y, w, f, d, av, m, ny, dtm);
 }
 
 template <class T>

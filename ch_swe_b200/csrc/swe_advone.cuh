@@ -2,12 +2,13 @@
 // vectors of points, the form of swe_onepass.cuh:
 //   k_adv_co2   contravariant components ut, vt (co2contra_Ch_mod.f90:27-94)
 //   k_adv_flux  J times the up4 mass flux on the u and v points (massflux_ch_mod.f90:80-121)
+//   k_adv_tend  up4 advection and Christoffel terms (vector_advection_Ch_mod.f90:33-115)
 //   k_adv_stage divergence of the flux with its SAT and scalar edge sync, gradient of the
 //               total depth, Coriolis with the vector edge sync, the advective tendencies and
 //               the RK4 update (operator_adv_swm_mod.f90:62-96, rk4_mod.f90:28-40)
 // A tile of k_adv_stage that touches a panel edge reads the neighbour panel's contravariant
 // components and flux beside the edge itself, so the stage needs no edge strips and no
-// edge-sync launch; k_havg, k_vhalo and k_advt (swe_advective.cuh) stay as they are.
+// edge-sync launch; k_havg and k_vhalo (swe_advective.cuh) stay as they are.
 #pragma once
 
 #include "swe_advective.cuh"
@@ -124,83 +125,287 @@ __global__ void __launch_bounds__(CoLayout<T, XL, TH>::NM)
 // ---------------------------------------------------------------------------
 // k_adv_flux: J F on the u (field 1) and v points (field 2), one vector of points per thread
 // ---------------------------------------------------------------------------
+// Blocks with blockIdx.y < ny take 8 rows of 32 vectors and every flux whose six points lie in
+// the panel.  The vectors beside columns 1 and n (u points) and the rows beside rows 1 and n
+// (v points) read virtual points interpolated along the neighbour's grid lines, a chain of
+// dependent loads: they are items of the further blocks, so that no other warp waits for them.
+__host__ __device__ __forceinline__ int flux_first_edge(int n, int VW)
+{
+    // the first vector whose six-point windows reach beyond column n
+    return n - VW - 3 < 0 ? 1 : ((n - VW - 3) / VW + 1 > 1 ? (n - VW - 3) / VW + 1 : 1);
+}
+__host__ __device__ __forceinline__ int flux_edge_items(int N, int VW)
+{
+    const int n = N + 1, NV = (n + VW - 1) / VW;
+    return n * (1 + NV - flux_first_edge(n, VW)) + 4 * NV;
+}
+
 template <class T>
 __global__ void __launch_bounds__(256) k_adv_flux(const T *__restrict__ Y, const T *__restrict__ W, T *__restrict__ F, Dims d,
-                                                  AdvView<T> av, MetricView<T> m, const double *__restrict__ dtm)
+                                                  AdvView<T> av, MetricView<T> m, int ny, const double *__restrict__ dtm)
 {
     using V = OV<T>;
     constexpr int VW = V::W;
-    const int N = d.N, n = N + 1, P = d.P, NV = (n + VW - 1) / VW;
+    const int N = d.N, n = N + 1, P = d.P, NV = (n + VW - 1) / VW, vre = flux_first_edge(n, VW);
     const int mem = blockIdx.z / NPAN, t = blockIdx.z % NPAN;
     if (member_frozen(dtm, mem)) return;
-    const int v = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y + 1, k = 1 + VW * v;
+    const int64_t po = mem * d.ms + t * d.ps;
+    const T *const h = Y + mem * d.ms;
     pdl_trigger();
-    const int64_t o = box_off(P, k, j), po = mem * d.ms + t * d.ps;
-    const bool ok = v < NV && j <= n;
-    V jy = ov_all(T(0)), jx = jy;
-    if (ok) {
-        jy = ov_ld(m.Jy + o);
-        jx = ov_ld(m.Jx + o);
-    }
-    pdl_wait();
-    if (!ok) return;
-    const T *h = Y + mem * d.ms, *hr = h + t * d.ps + o;
-    {
-        const V c = ov_ld(W + po + d.fs + o);
-        V f;
-        if (k >= 3 && k + VW - 1 <= N - 2) {
+    if ((int)blockIdx.y < ny) {
+        const int v = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y + 1, k = 1 + VW * v;
+        const int64_t o = box_off(P, k, j);
+        const bool ok = v < NV && j <= n, fx = ok && v >= 1 && v < vre, fy = ok && j >= 3 && j <= N - 2;
+        V jy = ov_all(T(0)), jx = jy;
+        if (fx) jy = ov_ld(m.Jy + o);
+        if (fy) jx = ov_ld(m.Jx + o);
+        pdl_wait();
+        const T *const hr = h + t * d.ps + o;
+        if (fx) {
+            const V a = ov_ld(hr - 4 + (VW == 2 ? 2 : 0)), c = ov_ld(W + po + d.fs + o);
             T w[VW + 5];   // h(k-2 .. k+VW+2)
+            w[0] = a.a[VW - 2];
+            w[1] = a.a[VW - 1];
 #pragma unroll
-            for (int q = 0; q < VW + 5; q++) w[q] = __ldg(hr + q - 2);
+            for (int q = 0; q < VW + 3; q++) w[q + 2] = __ldg(hr + q);
+            V f;
 #pragma unroll
             for (int e = 0; e < VW; e++) f.a[e] = up4_flux(c.a[e], w[e], w[e + 1], w[e + 2], w[e + 3], w[e + 4], w[e + 5]);
-        } else {
-#pragma unroll 1
-            for (int e = 0; e < VW; e++) {
-                const int i = k + e;
-                T r = T(0);
-                if (i <= N) {
-                    T w[6];
-#pragma unroll
-                    for (int q = 0; q < 6; q++) w[q] = h_ext(h, d, av, t, i - 2 + q, j);
-                    const T ce = e == 0 ? c.a[0] : (e == 1 ? c.a[1] : (e == 2 ? c.a[VW > 2 ? 2 : 0] : c.a[VW > 2 ? 3 : 0]));
-                    r = up4_flux(ce, w[0], w[1], w[2], w[3], w[4], w[5]);
-                }
-#pragma unroll
-                for (int q = 0; q < VW; q++)
-                    if (q == e) f.a[q] = r;
-            }
+            ov_st(F + po + d.fs + o, ov_mul(f, jy));
         }
-        ov_st(F + po + d.fs + o, ov_mul(f, jy));
-    }
-    if (j <= N) {
-        const V c = ov_ld(W + po + 2 * d.fs + o);
-        V f;
-        if (j >= 3 && j <= N - 2) {
-            V w[6];
+        if (fy) {
+            V g[6], f;
 #pragma unroll
-            for (int q = 0; q < 6; q++) w[q] = ov_ld(hr + (q - 2) * P);
+            for (int q = 0; q < 6; q++) g[q] = ov_ld(hr + (q - 2) * P);
+            const V c = ov_ld(W + po + 2 * d.fs + o);
 #pragma unroll
             for (int e = 0; e < VW; e++)
-                f.a[e] = up4_flux(c.a[e], w[0].a[e], w[1].a[e], w[2].a[e], w[3].a[e], w[4].a[e], w[5].a[e]);
-        } else {
-#pragma unroll 1
-            for (int e = 0; e < VW; e++) {
-                const int i = k + e;
-                T r = T(0);
-                if (i <= n) {
-                    T w[6];
+                f.a[e] = up4_flux(c.a[e], g[0].a[e], g[1].a[e], g[2].a[e], g[3].a[e], g[4].a[e], g[5].a[e]);
+            ov_st(F + po + 2 * d.fs + o, ov_mul(f, jx));   // (zeros beyond column n, where W holds zeros)
+        }
+        return;
+    }
+    pdl_wait();
+    const int q0 = ((blockIdx.y - ny) * gridDim.x + blockIdx.x) * 256 + threadIdx.y * 32 + threadIdx.x;
+    const int ex = 1 + NV - vre;
+    if (q0 < n * ex) {
+        const int j = 1 + q0 / ex, e = q0 % ex, v = e == 0 ? 0 : vre + e - 1, k = 1 + VW * v;
+        const int64_t o = box_off(P, k, j);
+        const V c = ov_ld(W + po + d.fs + o), jy = ov_ld(m.Jy + o);
+        T w[VW + 5];
 #pragma unroll
-                    for (int q = 0; q < 6; q++) w[q] = h_ext(h, d, av, t, i, j - 2 + q);
-                    const T ce = e == 0 ? c.a[0] : (e == 1 ? c.a[1] : (e == 2 ? c.a[VW > 2 ? 2 : 0] : c.a[VW > 2 ? 3 : 0]));
-                    r = up4_flux(ce, w[0], w[1], w[2], w[3], w[4], w[5]);
-                }
+        for (int q = 0; q < VW + 5; q++) w[q] = k + q - 2 <= n + 2 ? h_ext(h, d, av, t, k + q - 2, j) : T(0);
+        V f;
 #pragma unroll
-                for (int q = 0; q < VW; q++)
-                    if (q == e) f.a[q] = r;
+        for (int e2 = 0; e2 < VW; e2++) {
+            f.a[e2] = up4_flux(c.a[e2], w[e2], w[e2 + 1], w[e2 + 2], w[e2 + 3], w[e2 + 4], w[e2 + 5]);
+            if (k + e2 > N) f.a[e2] = T(0);
+        }
+        ov_st(F + po + d.fs + o, ov_mul(f, jy));
+    } else if (q0 < n * ex + 4 * NV) {
+        const int q1 = q0 - n * ex, r = q1 / NV, v = q1 % NV, k = 1 + VW * v, j = r < 2 ? 1 + r : N - 3 + r;   // rows 1, 2, N-1, N
+        const int64_t o = box_off(P, k, j);
+        const V c = ov_ld(W + po + 2 * d.fs + o), jx = ov_ld(m.Jx + o);
+        V f;
+#pragma unroll
+        for (int e = 0; e < VW; e++) {
+            f.a[e] = T(0);
+            if (k + e <= n) {
+                T w[6];
+#pragma unroll
+                for (int q = 0; q < 6; q++) w[q] = h_ext(h, d, av, t, k + e, j - 2 + q);
+                f.a[e] = up4_flux(c.a[e], w[0], w[1], w[2], w[3], w[4], w[5]);
             }
         }
         ov_st(F + po + 2 * d.fs + o, ov_mul(f, jx));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// k_adv_tend: A_u, A_v = up4 advection + Christoffel terms before the edge sync (k_advt's values)
+// ---------------------------------------------------------------------------
+template <class T, int XL, int TH>
+struct TendLayout {
+    using L = OneLayout<T, XL, TH>;
+    static constexpr int YG = TH + 3, NM = (XL * YG + 31) / 32 * 32;
+    static constexpr int XR = 6 * L::SLOT, WE = XR + (XROW_LEN + L::VW - 1) / L::VW * L::VW,
+                         BAR = WE + XROW_OPS * ONE_EDGES * ONE_TAPS * L::VW, TOTAL = BAR + L::VW;
+    static size_t bytes() { return (size_t)TOTAL * sizeof(T); }
+};
+
+// 12 |c| times the upwind derivative of f along c at the middle of f[0..6] (up4_diff: the sign
+// of c picks the stencil or its mirror, c times the sign is |c|)
+template <class T>
+__device__ __forceinline__ T up4_adv(T c, T f0, T f1, T f2, T f3, T f4, T f5, T f6)
+{
+    const bool p = c >= T(0);
+    const T a = p ? f4 : f2, b = p ? f2 : f4, e = p ? f1 : f5, g = p ? f0 : f6;
+    return fabs(c) * (T(3) * a + T(10) * f3 - T(18) * b + T(6) * e - g);
+}
+
+template <class T, int XL, int TH>
+__global__ void __launch_bounds__(TendLayout<T, XL, TH>::NM, 2)
+    k_adv_tend(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmW, const T *__restrict__ VH,
+               T *__restrict__ A, Dims d, AdvView<T> av, OneMetric<T> om, T inv_hxa, OneTiles ot, const double *__restrict__ dtm,
+               int *err)
+{
+    using C = TendLayout<T, XL, TH>;
+    using L = OneLayout<T, XL, TH>;
+    using V = OV<T>;
+    constexpr int VW = L::VW, HV = L::HV, SW = L::SW, NM = C::NM;
+    extern __shared__ __align__(128) unsigned char osm_raw[];
+    T *const sm = reinterpret_cast<T *>(osm_raw);
+    T *const sU = sm, *const sV = sm + L::SLOT, *const sUT = sm + 2 * L::SLOT, *const sVT = sm + 3 * L::SLOT,
+             *const sVH = sm + 4 * L::SLOT, *const sUH = sm + 5 * L::SLOT;
+    T *const xr = sm + C::XR, *const we = sm + C::WE;
+    uint64_t *const bar = reinterpret_cast<uint64_t *>(sm + C::BAR);
+    const int N = d.N, n = N + 1, P = d.P, NV = (n + VW - 1) / VW, bx = blockIdx.x, by = blockIdx.y;
+    const int t = blockIdx.z % NPAN, mem = blockIdx.z / NPAN;
+    if (member_frozen(dtm, mem)) return;
+    const int v0 = bx * ot.qx + min(bx, ot.rx), v1 = v0 + ot.qx + (bx < ot.rx);
+    const int i0 = 1 + VW * v0, i1 = min(1 + VW * v1, n + 1);
+    const int j0 = 1 + by * ot.qy + min(by, ot.ry), j1 = j0 + ot.qy + (by < ot.ry);
+    const int tid = threadIdx.x, rows = N + 1 + 2 * MG;
+    auto SI = [&](int i, int j) { return (j - j0 + 4) * SW + (i - i0 + 4); };
+    const unsigned touch = (i0 == 1 ? 1u : 0u) | (i1 == n + 1 ? 2u : 0u) | (j0 == 1 ? 4u : 0u) | (j1 == n + 1 ? 8u : 0u);
+    pdl_trigger();
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        fence_barrier_init();
+        mbar_arrive_expect_tx(bar, (uint32_t)(4 * L::BOX_BYTES));
+        pdl_wait();
+        const int yr = (mem * 3 * NPAN + t) * rows + (j0 - 1), fr = NPAN * rows;
+        tma_load_2d(sUT, &tmW, bar, i0 - 1, yr + fr);
+        tma_load_2d(sVT, &tmW, bar, i0 - 1, yr + 2 * fr);
+        tma_load_2d(sU, &tmY, bar, i0 - 1, yr + fr);
+        tma_load_2d(sV, &tmY, bar, i0 - 1, yr + 2 * fr);
+    }
+    const int tx = tid % XL, ty = tid / XL, k = i0 - 4 + VW * tx, j = j0 + ty;
+    const bool lane_ok = ty < C::YG, in_tile = lane_ok && tx >= HV && tx < HV + (v1 - v0), work = in_tile && j < j1;
+    int ve = -1, ec = 0, ei = 0;
+    {
+        const int v = v0 - HV + tx, vr = (n - 4) / VW;
+        if (v >= 0 && v < HV) { ve = v; ec = ei = 1 - k; }
+        else if (v >= vr && v < NV) { ve = HV + (v - vr); ec = N - 7 - k; ei = n - 7 - k; }
+    }
+    if (touch) {
+        for (int q = tid; q < XROW_LEN; q += NM) xr[q] = __ldg(om.xr + q);
+        for (int q = tid; q < XROW_OPS * ONE_EDGES * ONE_TAPS && (touch & 3u); q += NM)
+            ov_st(we + q * VW, *reinterpret_cast<const V *>(om.we + q * VW));
+    }
+    V g11 = ov_all(T(0)), g21 = g11, g22 = g11;
+    const int o = box_off32(P, k, j);
+    if (work) {
+        g11 = ov_ld(av.S + o);
+        g21 = ov_ld(av.S + d.ps + o);
+        g22 = ov_ld(av.S + 2 * d.ps + o);
+    }
+    __syncwarp();
+    if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
+        atomicExch(err, 1);
+        mbar_wait(bar, 0, FUSED_WAIT_NS);
+    }
+    __syncthreads();
+    // ---- vh = I_c2i,y(vt) on the tile's rows and the columns the i2c rows read; uh = I_c2i,x(ut)
+    // on the tile's columns and rows [j0-1, j1+2); the winds beyond the panel from the halo points
+    if (lane_ok && j < j1) ov_st(sVH + SI(k, j), one_y<0, false, SW>(sVT + SI(k, 0), (const T *)nullptr, j, n, xr));
+    {
+        const int m = max(j0 - 1, 1) + ty;
+        if (in_tile && m < min(j1 + 2, n + 1)) ov_st(sUH + SI(k, m), one_x<0>(sUT + SI(k, m), ve, ec, we));
+    }
+    if (touch) {
+        pdl_wait();
+        const T *const vh = VH + ((int64_t)mem * NPAN + t) * av.hp;
+        const int tw = i1 - i0, th = j1 - j0;
+        if (touch & 3u)
+            for (int q = tid; q < 3 * th; q += NM) {
+                const int c = q / th, l = j0 + q - c * th;   // c + 1 points beyond the panel
+                if (touch & 1u) {
+                    sU[SI(-c, l)] = vh[vh_u_w(N) + c * (N + 1) + (l - 1)];
+                    if (l <= N) sV[SI(-c, l)] = vh[vh_v_w(N) + c * N + (l - 1)];
+                }
+                if (touch & 2u) {
+                    sU[SI(N + 1 + c, l)] = vh[vh_u_e(N) + c * (N + 1) + (l - 1)];
+                    if (l <= N) sV[SI(N + 2 + c, l)] = vh[vh_v_e(N) + c * N + (l - 1)];
+                }
+            }
+        if (touch & 12u)
+            for (int q = tid; q < 3 * tw; q += NM) {
+                const int c = q / tw, i = i0 + q - c * tw;
+                if (touch & 4u) {
+                    if (i <= N) sU[SI(i, -c)] = vh[vh_u_s(N) + c * N + (i - 1)];
+                    sV[SI(i, -c)] = vh[vh_v_s(N) + c * (N + 1) + (i - 1)];
+                }
+                if (touch & 8u) {
+                    if (i <= N) sU[SI(i, N + 2 + c)] = vh[vh_u_n(N) + c * N + (i - 1)];
+                    sV[SI(i, N + 1 + c)] = vh[vh_v_n(N) + c * (N + 1) + (i - 1)];
+                }
+            }
+    }
+    __syncthreads();
+    if (!work) return;
+    const int64_t po = (int64_t)mem * d.ms + (int64_t)t * d.ps + o;
+    const int so = SI(k, j);
+    const T s2 = T(1.0 / ONE_IS), ca = -inv_hxa * T(1.0 / 12.0), cr = -av.inv_neg_radius;
+    // the tendency of one wind component f with the advecting (a, b) there
+    auto tend = [&](const T *f, const V &a, const V &b) {
+        T x[VW + 6];
+        {
+            T lo[VW == 4 ? 4 : 4], hi[4];
+            if constexpr (VW == 4) {
+                const V l = ov_ld(f - 4), r = ov_ld(f + 4);
+#pragma unroll
+                for (int e = 0; e < 4; e++) { lo[e] = l.a[e]; hi[e] = r.a[e]; }
+            } else {
+                const V l0 = ov_ld(f - 4), l1 = ov_ld(f - 2), r0 = ov_ld(f + 2), r1 = ov_ld(f + 4);
+                lo[0] = l0.a[0]; lo[1] = l0.a[1]; lo[2] = l1.a[0]; lo[3] = l1.a[1];
+                hi[0] = r0.a[0]; hi[1] = r0.a[1]; hi[2] = r1.a[0]; hi[3] = r1.a[1];
+            }
+            const V c = ov_ld(f);
+#pragma unroll
+            for (int e = 0; e < 3; e++) { x[e] = lo[e + 1]; x[VW + 3 + e] = hi[e]; }
+#pragma unroll
+            for (int e = 0; e < VW; e++) x[3 + e] = c.a[e];
+        }
+        V y[7], r;
+#pragma unroll
+        for (int q = 0; q < 7; q++) y[q] = ov_ld(f + (q - 3) * SW);
+#pragma unroll
+        for (int e = 0; e < VW; e++) {
+            const T ae = a.a[e], be = b.a[e];
+            const T s = up4_adv(ae, x[e], x[e + 1], x[e + 2], x[e + 3], x[e + 4], x[e + 5], x[e + 6]) +
+                        up4_adv(be, y[0].a[e], y[1].a[e], y[2].a[e], y[3].a[e], y[4].a[e], y[5].a[e], y[6].a[e]);
+            r.a[e] = s * ca + (ae * ae * g11.a[e] + T(2) * ae * be * g21.a[e] + be * be * g22.a[e]) * cr;
+        }
+        return r;
+    };
+    {
+        // u points: ut and v_at_u = I_i2c,x(vh)
+        V b = one_x<2>(sVH + so, ve, ei, we);
+#pragma unroll
+        for (int e = 0; e < VW; e++) b.a[e] *= s2 * s2;
+        V r = tend(sU + so, ov_ld(sUT + so), b);
+        if (k + VW > n)
+#pragma unroll
+            for (int e = 0; e < VW; e++)
+                if (k + e > N) r.a[e] = T(0);
+        ov_st(A + po + d.fs, r);
+    }
+    if (j <= N) {
+        // v points: u_at_v = I_i2c,y(uh) and vt
+        const T *S = av.S + 3 * d.ps + o;
+        g11 = ov_ld(S);
+        g21 = ov_ld(S + d.ps);
+        g22 = ov_ld(S + 2 * d.ps);
+        V a = one_y<2, false, SW>(sUH + SI(k, 0), (const T *)nullptr, j, N, xr);
+#pragma unroll
+        for (int e = 0; e < VW; e++) a.a[e] *= s2 * s2;
+        V r = tend(sV + so, a, ov_ld(sVT + so));
+        if (k + VW > n)
+#pragma unroll
+            for (int e = 0; e < VW; e++)
+                if (k + e > n) r.a[e] = T(0);
+        ov_st(A + po + 2 * d.fs, r);
     }
 }
 

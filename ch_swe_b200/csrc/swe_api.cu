@@ -1686,6 +1686,11 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
     auto co2 = [&] { AdvOneTU<T>::co2(c->olabel, c->oocc, M, tmY, (T *)c->w, c->dims, om, (const T *)c->fmet, dtm, c->derr, st); };
     auto havg = [&] { launch_k(k_havg<T>, hg, dim3(HAVG_THREADS), 0, sd, (T *)yin, (T *)c->hb, c->dims, dtm); };
     auto vhalo = [&] { launch_k(k_vhalo<T>, vg, dim3(256), 0, sd, (const T *)yin, (T *)c->vh, c->dims, av, M, dtm); };
+    auto tend = [&] {
+        if (!AdvOneTU<T>::tend(c->olabel, c->oocc, M, tmY, tmW, (const T *)c->vh, (T *)c->adt, c->dims, av, om, mv.inv_hxa, dtm,
+                               c->derr, sd))
+            launch_adv<T>(c, yin, av, mv, dtm, sd);
+    };
     auto flux = [&] { AdvOneTU<T>::flux(M, (const T *)yin, (const T *)c->w, (T *)c->fl, c->dims, av, mv, dtm, st); };
     if (fork) {
         // the averaging of h, the wind halo and the advective tendencies beside co2 and the flux
@@ -1697,7 +1702,7 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
         co2();
         cudaEventRecord(c->ev_co2, st);
         cudaStreamWaitEvent(sd, c->ev_co2, 0);
-        launch_adv<T>(c, yin, av, mv, dtm, sd);
+        tend();
         cudaEventRecord(c->ev_side, sd);
         cudaStreamWaitEvent(st, c->ev_havg, 0);
         flux();
@@ -1706,7 +1711,7 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
         co2();
         havg();
         vhalo();
-        launch_adv<T>(c, yin, av, mv, dtm, st);
+        tend();
         flux();
     }
     StageArgs a{mode, dt, c->ones, dtm, c->fl, c->adt, c->hb, c->hs};
