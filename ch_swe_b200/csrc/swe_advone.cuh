@@ -136,8 +136,8 @@ __host__ __device__ __forceinline__ int flux_first_edge(int n, int VW)
 }
 __host__ __device__ __forceinline__ int flux_edge_items(int N, int VW)
 {
-    const int n = N + 1, NV = (n + VW - 1) / VW;
-    return n * (1 + NV - flux_first_edge(n, VW)) + 4 * NV;
+    const int n = N + 1;
+    return n * (VW + n - VW * flux_first_edge(n, VW)) + 4 * n;
 }
 
 template <class T>
@@ -186,39 +186,28 @@ __global__ void __launch_bounds__(256) k_adv_flux(const T *__restrict__ Y, const
         return;
     }
     pdl_wait();
+    // one edge point per thread
     const int q0 = ((blockIdx.y - ny) * gridDim.x + blockIdx.x) * 256 + threadIdx.y * 32 + threadIdx.x;
-    const int ex = 1 + NV - vre;
-    if (q0 < n * ex) {
-        const int j = 1 + q0 / ex, e = q0 % ex, v = e == 0 ? 0 : vre + e - 1, k = 1 + VW * v;
-        const int64_t o = box_off(P, k, j);
-        const V c = ov_ld(W + po + d.fs + o), jy = ov_ld(m.Jy + o);
-        T w[VW + 5];
+    const int wx = VW + n - VW * vre, nx = n * wx;   // u points of a row: 1..VW and VW vre + 1 .. n
+    int i, j, f;
+    if (q0 < nx) {
+        f = 1;
+        j = 1 + q0 / wx;
+        i = 1 + q0 - (j - 1) * wx;
+        if (i > VW) i += VW * (vre - 1);
+        if (i > N) return;
+    } else if (q0 < nx + 4 * n) {
+        f = 2;
+        const int r = (q0 - nx) / n;
+        i = 1 + q0 - nx - r * n;
+        j = r < 2 ? 1 + r : N - 3 + r;               // v points of the rows 1, 2, N-1, N
+    } else return;
+    const int64_t o = box_off(P, i, j);
+    const T c = __ldg(W + po + f * d.fs + o), J = __ldg((f == 1 ? m.Jy : m.Jx) + o);
+    T w[6];
 #pragma unroll
-        for (int q = 0; q < VW + 5; q++) w[q] = k + q - 2 <= n + 2 ? h_ext(h, d, av, t, k + q - 2, j) : T(0);
-        V f;
-#pragma unroll
-        for (int e2 = 0; e2 < VW; e2++) {
-            f.a[e2] = up4_flux(c.a[e2], w[e2], w[e2 + 1], w[e2 + 2], w[e2 + 3], w[e2 + 4], w[e2 + 5]);
-            if (k + e2 > N) f.a[e2] = T(0);
-        }
-        ov_st(F + po + d.fs + o, ov_mul(f, jy));
-    } else if (q0 < n * ex + 4 * NV) {
-        const int q1 = q0 - n * ex, r = q1 / NV, v = q1 % NV, k = 1 + VW * v, j = r < 2 ? 1 + r : N - 3 + r;   // rows 1, 2, N-1, N
-        const int64_t o = box_off(P, k, j);
-        const V c = ov_ld(W + po + 2 * d.fs + o), jx = ov_ld(m.Jx + o);
-        V f;
-#pragma unroll
-        for (int e = 0; e < VW; e++) {
-            f.a[e] = T(0);
-            if (k + e <= n) {
-                T w[6];
-#pragma unroll
-                for (int q = 0; q < 6; q++) w[q] = h_ext(h, d, av, t, k + e, j - 2 + q);
-                f.a[e] = up4_flux(c.a[e], w[0], w[1], w[2], w[3], w[4], w[5]);
-            }
-        }
-        ov_st(F + po + 2 * d.fs + o, ov_mul(f, jx));
-    }
+    for (int q = 0; q < 6; q++) w[q] = h_ext(h, d, av, t, f == 1 ? i - 2 + q : i, f == 1 ? j : j - 2 + q);
+    F[po + f * d.fs + o] = up4_flux(c, w[0], w[1], w[2], w[3], w[4], w[5]) * J;
 }
 
 // ---------------------------------------------------------------------------
