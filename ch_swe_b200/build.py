@@ -28,7 +28,7 @@ ONE_SOURCES = ["one_f.cu", "one_d.cu"]
 ADVONE_SOURCES = ["advone_f.cu", "advone_d.cu"]
 SOURCES = ["swe_api.cu", *STAGE_SOURCES, *FUSED_SOURCES, *GROUP_SOURCES, *ONE_SOURCES, *ADVONE_SOURCES]
 COMMON_HEADERS = ["swe_common.cuh", "swe_kernels.cuh", "swe_sbp.cuh", "sbp63.h", "swe_advective.cuh", "swe_launch.cuh",
-                  "swe_fused.cuh", "swe_tma.cuh"]
+                  "swe_fused.cuh", "swe_tma.cuh", "swe_vec.cuh"]
 UNIT_HEADERS = {"swe_api.cu": COMMON_HEADERS + ["swe_ah.cuh", "swe_cgrid.cuh", "swe_diff.cuh", "lap63.h", "swe_one_launch.cuh",
                                                 "swe_adv_launch.cuh"],
                 **{src: COMMON_HEADERS + ["fused_tu.cuh"] for src in FUSED_SOURCES},

@@ -2431,16 +2431,18 @@ static int enqueue_diffusion(swe_ctx *c, T *y, T *out, double dt, const double *
     const T *mb42 = (const T *)c->dif_b + (size_t)NPAN * 6 * d.ps, *mb63 = mb42 + (size_t)2 * n * 2 * 48;
     const T *w21 = mb63 + (size_t)2 * n * 2 * 108, *w42 = w21 + (size_t)2 * 3 * d.ps, *w63 = w42 + (size_t)2 * 5 * d.ps;
     const DifView<T> dv{(const T *)c->dif_b, mb42, mb63, w21, w42, w63, hxa * hxa};
-    const dim3 pb(32, 8), pm((n + 31) / 32, (n + 7) / 8, NPAN * M), pf((n + 31) / 32, (n + 7) / 8, NPAN * M * DIF_FIELDS);
+    const dim3 pb(32, 8), pm((n + 31) / 32, (n + 7) / 8, NPAN * M);
     const dim3 sg((4 * N + 255) / 256, 1, NPAN * M * DIF_FIELDS);
     launch_k(k_dif_prep<T>, pm, pb, 0, c->stream, (const T *)y, X, d, dv);
     // L(X) -> A, then L(A) -> X
+    const DifSplit sp = dif_split(N, lap_order, OV<T>::W);
+    const dim3 pf(sp.ni + sp.ne, 1, NPAN * M * (DIF_FIELDS / DIF_PAIR));
     T *src = X, *dst = A;
     for (int pass = 0; pass < 2; pass++) {
-        launch_k(lap_order == 63 ? k_dif_d1<T, 63> : (lap_order == 42 ? k_dif_d1<T, 42> : k_dif_d1<T, 21>), pf, pb, 0,
-                 c->stream, (const T *)src, D1X, D1Y, d, av);
-        launch_k(lap_order == 63 ? k_dif_lap<T, 63> : (lap_order == 42 ? k_dif_lap<T, 42> : k_dif_lap<T, 21>), pf, pb, 0,
-                 c->stream, (const T *)src, (const T *)D1X, (const T *)D1Y, R, dst, d, av, dv);
+        launch_k(lap_order == 63 ? k_dif_d1<T, 63> : (lap_order == 42 ? k_dif_d1<T, 42> : k_dif_d1<T, 21>), pf,
+                 dim3(256), 0, c->stream, (const T *)src, D1X, D1Y, d, av, sp);
+        launch_k(lap_order == 63 ? k_dif_lap<T, 63> : (lap_order == 42 ? k_dif_lap<T, 42> : k_dif_lap<T, 21>), pf,
+                 dim3(256), 0, c->stream, (const T *)src, (const T *)D1X, (const T *)D1Y, R, dst, d, av, dv, sp);
         launch_k(k_dif_sync<T>, sg, dim3(256), 0, c->stream, (const T *)R, dst, d);
         std::swap(src, dst);
     }

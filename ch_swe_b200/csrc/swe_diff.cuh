@@ -24,6 +24,7 @@
 
 #include "lap63.h"
 #include "swe_ah.cuh"
+#include "swe_vec.cuh"
 
 namespace chswe {
 
@@ -183,66 +184,232 @@ __global__ void __launch_bounds__(256) k_dif_prep(const T *__restrict__ Y, T *__
         X[dif_base(d, mem, 1 + k) + t * d.ps + o] = b[k * d.ps] * u + b[(3 + k) * d.ps] * w;
 }
 
+// Split of a panel's n x n vertices for the difference passes: the vectors (swe_vec.cuh)
+// whose points and rows all take interior rows of both the narrow second difference and the
+// first difference, and the remaining vertices, one per thread.  The two parts are blocks
+// of their own: a warp never waits for closure rows beside its interior points.
+struct DifSplit {
+    int n, va, nv, lo, nr;   // first vector, vectors per row, first row, rows; nv * nr == 0: none
+    int ni, ne;              // blocks of the interior vectors and of the other vertices
+};
+__host__ __device__ constexpr int dif_lo(int ord) { return ord == 21 ? 2 : (ord == 42 ? 7 : 10); }
+static inline DifSplit dif_split(int N, int ord, int VW)
+{
+    DifSplit s{};
+    const int n = N + 1, lo = dif_lo(ord), hi = n + 1 - lo;
+    s.n = n;
+    s.lo = lo;
+    s.va = (lo - 1 + VW - 1) / VW;
+    s.nv = hi / VW - s.va;
+    s.nr = hi - lo + 1;
+    if (s.nv < 1 || s.nr < 1) s.nv = s.nr = 0;
+    s.ni = (s.nv * s.nr + 255) / 256;
+    s.ne = (n * n - s.nv * VW * s.nr + 255) / 256;
+    return s;
+}
+// Vertex q of those outside the interior vectors; false past the last.
+template <int VW>
+__device__ __forceinline__ bool dif_edge_vertex(const DifSplit &s, int q, int &i, int &j)
+{
+    const int n = s.n;
+    if (s.nr == 0) {
+        if (q >= n * n) return false;
+        j = q / n;
+        i = q - j * n + 1;
+        j++;
+        return true;
+    }
+    const int rows = n - s.nr, top = rows * n;    // the rows below and above the interior rows
+    if (q < top) {
+        j = q / n;
+        i = q - j * n + 1;
+        j = j < s.lo - 1 ? j + 1 : j + 1 + s.nr;
+        return true;
+    }
+    const int w = n - s.nv * VW;                  // the columns beside the interior vectors
+    q -= top;
+    if (q >= w * s.nr) return false;
+    j = q / w;
+    i = q - j * w + 1;
+    j += s.lo;
+    if (i > s.va * VW) i += s.nv * VW;
+    return true;
+}
+// x[q] = f(k - R + q), q = 0 .. VW + 2 R - 1, around the vector at p
+template <class T, int R>
+__device__ __forceinline__ void dif_row(const T *p, T (&x)[OV<T>::W + 2 * R])
+{
+    constexpr int VW = OV<T>::W, H = (R + VW - 1) / VW;   // vectors beside the own one
+    OV<T> v[2 * H + 1];
+#pragma unroll
+    for (int m = 0; m < 2 * H + 1; m++) v[m] = ov_ld(p + (m - H) * VW);
+#pragma unroll
+    for (int q = 0; q < VW + 2 * R; q++) x[q] = v[(q - R + H * VW) / VW].a[(q - R + H * VW) % VW];
+}
+// The interior row of the node difference of order ORD on f(k - R .. k + R) (dn2n's).
+template <class T, int ORD>
+__device__ __forceinline__ T dif_d1_in(const T *f)
+{
+    if constexpr (ORD == 21) return (-f[0] + f[2]) / T(2);
+    else if constexpr (ORD == 42) return (f[0] + T(-8) * f[1] + T(8) * f[3] + -f[4]) / T(12);
+    else return (-f[0] + T(9) * f[1] + T(-45) * f[2] + T(45) * f[4] + T(-9) * f[5] + f[6]) / T(60);
+}
+constexpr int DIF_PAIR = 2;   // fields per thread of the interior vectors: the metric is read once for both
+
 // calc_tile_d1x_d1y: d1x = D1x(f) J Qi12, d1y = D1y(f) J Qi12 (sbp_diff_<ORD> node
-// differences).  Grid z: panel + NPAN * (field + 4 member).
+// differences).  Grid x: interior blocks, then the others; z: panel + NPAN * (field pair +
+// 2 member).  The point-wise kernel read every stencil input of every vertex by itself
+// (18 loads per vertex and field with the Laplacian's, 13 us per launch at C192 FP32 cold).
 template <class T, int ORD>
 __global__ void __launch_bounds__(256) k_dif_d1(const T *__restrict__ F, T *__restrict__ D1X, T *__restrict__ D1Y, Dims d,
-                                                AhView<T> a)
+                                                AhView<T> a, DifSplit sp)
 {
-    const int n = d.N + 1;
-    const int t = blockIdx.z % NPAN;
-    const int64_t base = (int64_t)(blockIdx.z / NPAN) * NPAN * d.ps + t * d.ps;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+    using V = OV<T>;
+    constexpr int VW = V::W, R = (ORD == 21 ? 1 : (ORD == 42 ? 2 : 3));
+    const int n = d.N + 1, P = d.P, t = blockIdx.z % NPAN;
+    const int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_PAIR * NPAN * d.ps + t * d.ps;
     pdl_trigger();
+    if ((int)blockIdx.x < sp.ni) {
+        const int q = blockIdx.x * 256 + threadIdx.x;
+        const bool ok = q < sp.nv * sp.nr;
+        const int r = ok ? q / sp.nv : 0, v = sp.va + q - r * sp.nv, j = sp.lo + r;
+        const int64_t o = ok ? box_off(P, 1 + VW * v, j) : 0;
+        V J = ov_all(T(0)), Q2 = J;
+        if (ok) {
+            J = ov_ld(a.J + o);
+            Q2 = ov_ld(a.Q2 + o);
+        }
+        pdl_wait();
+        if (!ok) return;
+#pragma unroll
+        for (int fl = 0; fl < DIF_PAIR; fl++) {
+            const int64_t b = base + (int64_t)fl * NPAN * d.ps + o;
+            const T *f = F + b;
+            T x[VW + 2 * R];
+            dif_row<T, R>(f, x);
+            V y[2 * R + 1], ox, oy;
+#pragma unroll
+            for (int m = 0; m < 2 * R + 1; m++) y[m] = ov_ld(f + (m - R) * P);
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                T c[2 * R + 1];
+#pragma unroll
+                for (int m = 0; m < 2 * R + 1; m++) c[m] = y[m].a[e];
+                ox.a[e] = dif_d1_in<T, ORD>(x + e) * J.a[e] * Q2.a[e];
+                oy.a[e] = dif_d1_in<T, ORD>(c) * J.a[e] * Q2.a[e];
+            }
+            ov_st(D1X + b, ox);
+            ov_st(D1Y + b, oy);
+        }
+        return;
+    }
     pdl_wait();
-    if (i > n || j > n) return;
-    const GV<T> f{F + base, d.P};
-    const int64_t o = box_off(d.P, i, j);
+    int i, j;
+    if (!dif_edge_vertex<VW>(sp, ((int)blockIdx.x - sp.ni) * 256 + threadIdx.x, i, j)) return;
+    const int64_t o = box_off(P, i, j);
     const T J = __ldg(a.J + o), Q2 = __ldg(a.Q2 + o);
-    D1X[base + o] = dn2n<T, ORD>(i, n, [&](int k) { return f(k, j); }) * J * Q2;
-    D1Y[base + o] = dn2n<T, ORD>(j, n, [&](int l) { return f(i, l); }) * J * Q2;
+#pragma unroll
+    for (int fl = 0; fl < DIF_PAIR; fl++) {
+        const int64_t b = base + (int64_t)fl * NPAN * d.ps;
+        const GV<T> f{F + b, P};
+        D1X[b + o] = dn2n<T, ORD>(i, n, [&](int k) { return f(k, j); }) * J * Q2;
+        D1Y[b + o] = dn2n<T, ORD>(j, n, [&](int l) { return f(i, l); }) * J * Q2;
+    }
 }
 
 // calc_laplace_tile and divide_by_J_self: the panel-local Laplacian of every vertex; the
-// panel-boundary vertices' values go to R (for the sync), the others to OUT.
+// panel-boundary vertices' values go to R (for the sync), the others to OUT.  The same grid.
 template <class T, int ORD>
 __global__ void __launch_bounds__(256) k_dif_lap(const T *__restrict__ F, const T *__restrict__ D1X,
-                                                 const T *__restrict__ D1Y, T *__restrict__ R, T *__restrict__ OUT, Dims d,
-                                                 AhView<T> a, DifView<T> v)
+                                                 const T *__restrict__ D1Y, T *__restrict__ RAW, T *__restrict__ OUT, Dims d,
+                                                 AhView<T> a, DifView<T> v, DifSplit sp)
 {
-    const int n = d.N + 1;
-    const int t = blockIdx.z % NPAN;
-    const int64_t base = (int64_t)(blockIdx.z / NPAN) * NPAN * d.ps + t * d.ps;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+    using V = OV<T>;
+    constexpr int VW = V::W, R = (ORD == 21 ? 1 : (ORD == 42 ? 2 : 3));
+    const int n = d.N + 1, P = d.P, t = blockIdx.z % NPAN;
+    const int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_PAIR * NPAN * d.ps + t * d.ps;
+    const T *const w0 = ORD == 21 ? v.w21 : (ORD == 42 ? v.w42 : v.w63);
+    const int64_t wd = (int64_t)narrow_width(ORD) * d.ps;   // the y weights follow the x weights
     pdl_trigger();
+    if ((int)blockIdx.x < sp.ni) {
+        const int q = blockIdx.x * 256 + threadIdx.x;
+        const bool ok = q < sp.nv * sp.nr;
+        const int r = ok ? q / sp.nv : 0, vv = sp.va + q - r * sp.nv, j = sp.lo + r;
+        const int64_t o = ok ? box_off(P, 1 + VW * vv, j) : 0;
+        V wx[2 * R + 1], wy[2 * R + 1], J = ov_all(T(1));
+        if (ok) {
+#pragma unroll
+            for (int m = 0; m < 2 * R + 1; m++) {
+                wx[m] = ov_ld(w0 + m * d.ps + o);
+                wy[m] = ov_ld(w0 + wd + m * d.ps + o);
+            }
+            J = ov_ld(a.J + o);
+        }
+        pdl_wait();
+        if (!ok) return;
+#pragma unroll
+        for (int fl = 0; fl < DIF_PAIR; fl++) {
+            const int64_t b = base + (int64_t)fl * NPAN * d.ps + o;
+            const T *f = F + b;
+            T x[VW + 2 * R], z[VW + 2 * R];
+            dif_row<T, R>(f, x);
+            dif_row<T, R>(D1Y + b, z);
+            V y[2 * R + 1], u[2 * R + 1], out;
+#pragma unroll
+            for (int m = 0; m < 2 * R + 1; m++) {
+                y[m] = ov_ld(f + (m - R) * P);
+                u[m] = ov_ld(D1X + b + (m - R) * P);
+            }
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                T d2x = wx[0].a[e] * x[e], d2y = wy[0].a[e] * y[0].a[e], c[2 * R + 1];
+#pragma unroll
+                for (int m = 1; m < 2 * R + 1; m++) {
+                    d2x = d2x + wx[m].a[e] * x[e + m];
+                    d2y = d2y + wy[m].a[e] * y[m].a[e];
+                }
+#pragma unroll
+                for (int m = 0; m < 2 * R + 1; m++) c[m] = u[m].a[e];
+                T s = d2x + d2y;
+                s = s + dif_d1_in<T, ORD>(z + e) + dif_d1_in<T, ORD>(c);
+                out.a[e] = s / T(v.h2) / J.a[e];
+            }
+            ov_st(OUT + b, out);
+        }
+        return;
+    }
     pdl_wait();
-    if (i > n || j > n) return;
-    const GV<T> f{F + base, d.P}, dx1{D1X + base, d.P}, dy1{D1Y + base, d.P};
-    const GV<T> J{a.J, d.P}, Q1{a.Q1, d.P}, Q3{a.Q3, d.P};
+    int i, j;
+    if (!dif_edge_vertex<VW>(sp, ((int)blockIdx.x - sp.ni) * 256 + threadIdx.x, i, j)) return;
     // one end's closure block
     constexpr int RC = ORD == 63 ? NarrowBlock<63>::R * NarrowBlock<63>::C : NarrowBlock<42>::R * NarrowBlock<42>::C;
     const T *mb = ORD == 63 ? v.m63 : v.m42;
-    const T *wi = (ORD == 21 ? v.w21 : (ORD == 42 ? v.w42 : v.w63)) + box_off(d.P, i, j);
-    const int64_t wd = (int64_t)narrow_width(ORD) * d.ps;   // the y weights follow the x weights
-    T d2x = narrow_d2<T, ORD>(i, n, [&](int k) { return Q1(k, j) * J(k, j); }, [&](int k) { return f(k, j); },
-                              mb + dif_block_index(n, 0, j, 0, RC), wi, d.ps);
-    const T d2y = narrow_d2<T, ORD>(j, n, [&](int l) { return Q3(i, l) * J(i, l); }, [&](int l) { return f(i, l); },
-                                    mb + dif_block_index(n, 1, i, 0, RC), wi + wd, d.ps);
-    // the boundary penalties 1/h_1 (-+2 d1f), all on d2f_x and in the reference's order
-    const T pen = ORD == 21 ? T(2) : (ORD == 42 ? T(48.0 / 17) : T(43200.0 / 13649));
-    if (i == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dy1(1, j)));
-    if (i == n) d2x = d2x - T(0.5) * (pen * (T(2) * dy1(n, j)));
-    if (j == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dx1(i, 1)));
-    if (j == n) d2x = d2x - T(0.5) * (pen * (T(2) * dx1(i, n)));
-    const T dyx = dn2n<T, ORD>(j, n, [&](int l) { return dx1(i, l); });
-    const T dxy = dn2n<T, ORD>(i, n, [&](int k) { return dy1(k, j); });
-    T r = d2x + d2y;
-    r = r + dxy + dyx;
-    r = r / T(v.h2);
-    r = r / J(i, j);
-    const int64_t o = box_off(d.P, i, j);
-    if (i == 1 || i == n || j == 1 || j == n) R[base + o] = r;
-    else OUT[base + o] = r;
+    const T *wi = w0 + box_off(P, i, j);
+    const GV<T> J{a.J, P}, Q1{a.Q1, P}, Q3{a.Q3, P};
+#pragma unroll 1
+    for (int fl = 0; fl < DIF_PAIR; fl++) {
+        const int64_t b = base + (int64_t)fl * NPAN * d.ps;
+        const GV<T> f{F + b, P}, dx1{D1X + b, P}, dy1{D1Y + b, P};
+        T d2x = narrow_d2<T, ORD>(i, n, [&](int k) { return Q1(k, j) * J(k, j); }, [&](int k) { return f(k, j); },
+                                  mb + dif_block_index(n, 0, j, 0, RC), wi, d.ps);
+        const T d2y = narrow_d2<T, ORD>(j, n, [&](int l) { return Q3(i, l) * J(i, l); }, [&](int l) { return f(i, l); },
+                                        mb + dif_block_index(n, 1, i, 0, RC), wi + wd, d.ps);
+        // the boundary penalties 1/h_1 (-+2 d1f), all on d2f_x and in the reference's order
+        const T pen = ORD == 21 ? T(2) : (ORD == 42 ? T(48.0 / 17) : T(43200.0 / 13649));
+        if (i == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dy1(1, j)));
+        if (i == n) d2x = d2x - T(0.5) * (pen * (T(2) * dy1(n, j)));
+        if (j == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dx1(i, 1)));
+        if (j == n) d2x = d2x - T(0.5) * (pen * (T(2) * dx1(i, n)));
+        const T dyx = dn2n<T, ORD>(j, n, [&](int l) { return dx1(i, l); });
+        const T dxy = dn2n<T, ORD>(i, n, [&](int k) { return dy1(k, j); });
+        T r = d2x + d2y;
+        r = r + dxy + dyx;
+        r = r / T(v.h2);
+        r = r / J(i, j);
+        const int64_t o = box_off(P, i, j);
+        if (i == 1 || i == n || j == 1 || j == n) RAW[b + o] = r;
+        else OUT[b + o] = r;
+    }
 }
 
 // The Ah scalar sync of the panel-boundary vertices (halo_Ah_scalar_sync_mod.f90:43-98):

@@ -3,15 +3,9 @@
 #pragma once
 
 #include "swe_launch.cuh"
+#include "swe_vec.cuh"
 
 namespace chswe {
-
-// A 16-byte vector of T.
-template <class T>
-struct alignas(16) OV {
-    static constexpr int W = 16 / (int)sizeof(T);
-    T a[W];
-};
 
 // Per panel side, along the side (k_one_tables): JQ12 at across nodes 1..5 (lines 0-4), J Qn at
 // across centres 1..3 (5-7) and 1/J there (8-10), J Qt and 1/J on the edge line (11, 12).
