@@ -8,8 +8,8 @@
 namespace chswe {
 
 // Configurations of k_adv_stage and k_adv_co2: (label, XL, TH, blocks per SM, registers).
-#define CHSWE_ADVONE_CFGS_F(X) X(25, 10, 21, 2, 64) X(33, 10, 29, 2, 64)
-#define CHSWE_ADVONE_CFGS_D(X) X(17, 16, 15, 2, 64) X(25, 16, 23, 1, 96)
+#define CHSWE_ADVONE_CFGS_F(X) X(25, 10, 21, 2, 64) X(33, 9, 28, 2, 72)
+#define CHSWE_ADVONE_CFGS_D(X) X(17, 16, 15, 2, 64) X(25, 18, 25, 1, 96)
 
 template <class T>
 struct AdvOneTU {
