@@ -8,8 +8,8 @@
 namespace chswe {
 
 // Configurations of k_adv_stage and k_adv_co2: (label, XL, TH, blocks per SM, registers).
-#define CHSWE_ADVONE_CFGS_F(X) X(25, 10, 21, 2, 64) X(33, 9, 28, 2, 72)
-#define CHSWE_ADVONE_CFGS_D(X) X(17, 16, 15, 2, 64) X(25, 18, 25, 1, 96)
+#define CHSWE_ADVONE_CFGS_F(X) X(25, 15, 18, 2, 72) X(33, 9, 28, 2, 72)
+#define CHSWE_ADVONE_CFGS_D(X) X(17, 18, 14, 2, 72) X(25, 14, 18, 2, 72) X(33, 18, 28, 1, 80)
 
 template <class T>
 struct AdvOneTU {

@@ -1099,14 +1099,16 @@ static int alloc_box(swe_ctx *c, void **p)
 template <class T>
 static cudaError_t stage_smem_optin();
 
-// The one-launch configuration a linear Ch 4-2 context starts with; tile 0: the split
-// kernels.  Cubes below 16 cells keep the split kernels and their twelve launches a step,
-// which swe_launch_count reports there.  FP32 starts with the large tiles (measured per RK4
-// step at C24 / C48 / C96 / C192: 24 / 27 / 28 / 33 us against 85 / 75 / 80 / 86 us split).
-// FP64: the one-block-per-SM tiles where the grid fits one wave (C24 / C48 / C96: 23 / 24 /
-// 33 against 97 / 91 / 96 us split); where it does not, their advantage shrinks (C192: 83
-// against 102 us) and small cubes with many members are faster split (64 x C48: 496 against
-// 425 us: every tile holds a panel corner).
+// The vector stage's configuration a Ch 4-2 context starts with; tile 0: the split kernels.
+// Cubes below 16 cells keep the split kernels and their twelve launches a step, which
+// swe_launch_count reports there.
+//   FP32: tiles of 7 vectors by 28 rows at every size (measured per RK4 step, alone: C48 / C96 /
+//   C192 / C384 19.9 / 22.6 / 30.6 / 97.5 us against 75 / 80 / 86 / 176 us of the best split or
+//   fused configuration; 256 x C48 576 against 1139 us).
+//   FP64: full-width tiles for many members of a cube that one tile spans (64 x C48: 318 us
+//   against 371 with the large tiles and 425 split: fewer panel corners per block); tiles of 10
+//   vectors by 25 rows where they make at most one wave (C96: 27.4 against 29.0 us); else 14
+//   vectors by 28 rows (C192 69 against 102 us split, C384 213 against 265 us fused).
 template <class T>
 static KernelCfg one_default_cfg(int N, int members, bool adv)
 {
@@ -1114,15 +1116,18 @@ static KernelCfg one_default_cfg(int N, int members, bool adv)
     const KernelCfg none{0, 0, 0};
     if (N < 16) return none;
     if (adv) {
-        const KernelCfg k = sizeof(T) == 4 ? KernelCfg{33, 2, 3} : KernelCfg{17, 2, 3};
+        // FP64, alone, per RK4 step with (17, 2) / (25, 2) / (33, 1): C96 104 / 99 / 101 us, C192
+        // 171 / 197 / 159, C384 407 / 432 / 431
+        const KernelCfg k = sizeof(T) == 4 ? KernelCfg{33, 2, 3}
+                                           : (N < 128 ? KernelCfg{25, 2, 3} : (N < 256 ? KernelCfg{33, 1, 3} : KernelCfg{17, 2, 3}));
         return AdvOneTU<T>::grid(k.tile, k.occ, N, members, og) ? k : none;
     }
     if (sizeof(T) == 4) return OneTU<T>::grid(33, 2, N, members, og) ? KernelCfg{33, 2, 3} : none;
-    if (N < 128 && members > 4) return none;
+    if (members > 4 && OneTU<T>::grid(17, 1, N, members, og) && og.g.x == 1) return KernelCfg{17, 1, 3};
     for (int label : {25, 33})
         if (OneTU<T>::grid(label, 1, N, members, og) && (og.g.x * og.g.y * og.g.z <= 148 || label == 33))
             return KernelCfg{label, 1, 3};
-    return OneTU<T>::grid(17, 2, N, members, og) ? KernelCfg{17, 2, 3} : none;
+    return none;
 }
 
 extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)

@@ -73,8 +73,8 @@ static inline void one_edge_table(int N, int VW, double *we)
 
 // Configurations: (label, XL, TH, blocks per SM, registers per thread).  The label is the
 // public tile size, at least the rows of the configuration's tiles.
-#define CHSWE_ONE_CFGS_F(X) X(17, 16, 16, 2, 64) X(25, 16, 25, 1, 80) X(25, 10, 22, 2, 64) X(33, 9, 28, 2, 72)
-#define CHSWE_ONE_CFGS_D(X) X(17, 16, 16, 2, 64) X(25, 16, 22, 1, 96) X(33, 18, 28, 1, 80)
+#define CHSWE_ONE_CFGS_F(X) X(17, 15, 14, 2, 72) X(25, 15, 18, 2, 64) X(33, 9, 28, 2, 72)
+#define CHSWE_ONE_CFGS_D(X) X(17, 29, 17, 1, 72) X(25, 14, 25, 1, 96) X(33, 18, 28, 1, 80)
 
 // Balanced tiles: the first rx (ry) tiles hold qx + 1 vectors (qy + 1 rows), the others qx (qy).
 struct OneTiles {
