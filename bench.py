@@ -207,7 +207,8 @@ def measured_peaks():
 
 def profile_traffic(key):
     """DRAM bytes per launch of the stage kernel at C192 from the ncu captures summarised
-    under profiles/: key "fp32" (the split k_stage) or "fp32_fused" (k_fstage)."""
+    under profiles/: key "fp32" (the split k_stage), "fp32_fused" (k_fstage) or "fp32_vector"
+    (k_onepass)."""
     p = os.path.join(ROOT, "profiles", "k_stage_c192_traffic.json")
     if os.path.exists(p):
         try:
@@ -647,8 +648,10 @@ def run_ours(args):
     # the stage kernel of the configuration the autotuner chose: the split k_stage (its
     # contravariant components from k_co2contra) or the fused k_fstage (TMA tiles, the
     # contravariant components computed in the tile, edge strips from k_strip)
-    fused32 = r32["kernel_config"][2] == 2
-    kn = ("k_strip", "k_edge", "k_fstage") if fused32 else ("k_co2contra", "k_edge", "k_stage")
+    # or the one-launch k_onepass (nothing before it)
+    runs32 = r32["kernel_config"][2]
+    kn = {2: ("k_strip", "k_edge", "k_fstage"), 3: ("k_co2contra", "k_edge", "k_onepass")}.get(
+        runs32, ("k_co2contra", "k_edge", "k_stage"))
     peak = float(peaks.get("hbm_gbs", 6650.0))
     line = {
         "metric": "C192 RK4 cell-updates/s", "value": v32, "unit": "cell-updates/s", "n_gpus": world,
@@ -671,7 +674,7 @@ def run_ours(args):
                 "d2h_bytes_per_step": r32["e2e_bytes"],
                 "path": "ch_swe_b200.swm -> libchswe.so C ABI: upload (pinned staging), 576 RK4 steps, download"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": profile_traffic("fp32_fused" if fused32 else "fp32"), "kernel": kn[2] + "<float>",
+                     "traffic": profile_traffic({2: "fp32_fused", 3: "fp32_vector"}.get(runs32, "fp32")), "kernel": kn[2] + "<float>",
                      "peak_source": src, "ms_per_launch": r32["ms_stage"],
                      "alg_bytes_per_launch": alg_bytes_32},
         "gpu_launches": r32["launches"],

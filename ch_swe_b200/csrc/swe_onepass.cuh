@@ -13,10 +13,27 @@
 // points).  Point (i, j) of a panel box lies at column i + 3, so vector v holds the points
 // VW v + 1 .. VW v + VW and is 16-byte aligned in global and in shared memory.  A block
 // owns a tile of up to XL - 2 HV vectors by TH rows; its windows (h, u, v and seven metric
-// boxes, the tile plus four points on every side) come by TMA.  Thread (x, y) of the block
-// takes window vector x and a run of consecutive rows in every pass: y stencils slide a
-// window of four vectors down the run, x stencils read the own vector and the two or three
-// points beside it.
+// boxes, the tile plus four points on every side) come by TMA.  Main thread (x, y) takes
+// window vector x and row y of every pass: y stencils read four vectors of the column, x
+// stencils the own vector and the three points beside it.  ONE_BAND further threads per
+// touched side carry the boundary through loads, contravariant components and syncs beside
+// the passes and meet the main threads twice (named barriers): for the own panel's copies
+// after P2, and before P4.
+//
+// What bounds it, and why it has this shape (B200, C192 FP32 unless said otherwise).  The
+// former stage was three dependent launches (edge strips or contravariant components, edge
+// sync, tiles), about 21 us at any cube size up to C192, of which the kernels' own work was
+// under half: an RK4 step took 86 us, C24 55 us.  One launch takes 7.6 us per stage (30.6 us
+// per step; 22.3 us per step with three contexts at once).  A first version with 192 threads
+// per block, two rows per thread and the boundary as a loop of the same threads ran 17 us per
+// stage even at C24: the boundary's chain of dependent loads stood in the passes' way; its
+// threads of their own brought C24 to 6 us.  A stage's time now is one memory round trip for the
+// windows (0.8 us), four passes of 0.4 to 0.9 us and the RK4 stores; ncu counts 22 % of the L2
+// and 62 % of the shared-memory throughput at C384, issue slots 35 to 45 % busy: latency and
+// shared-memory traffic, not arithmetic (three instead of four operations per stencil and
+// packed FP32 changed nothing at C192).  Assigning the vectors of a pass to threads one after
+// another, without idle lanes, saved 14 % of the instructions and ran 5 to 25 % slower: the
+// rows' ends conflict in shared memory and fewer warps hide the latency.
 //
 // Ranges of the passes (x; y is symmetric) for tile [i0, i1), clipped to the panel:
 //   vq  = JQ12 I_c2i,y(v)          nodes   [i0-3, i1+3)
@@ -38,6 +55,10 @@ namespace chswe {
 // XL: window vectors per row; TH: maximal tile rows.  Main threads: XL x YG, one window row
 // each in every pass (YG >= TH + 6, the rows of the widest pass), whole warps; then
 // ONE_BAND threads per touched panel side, one per along-edge point of its band.
+// The shape decides more than anything else: it has to divide the panels without a remainder
+// wave or idle lanes.  FP32 7 x 28 (XL 9) against 8 x 30 (XL 10), per RK4 step: C192 30.6 /
+// 33.4 us (294 blocks, two per SM, either way), 256 x C48 577 / 639; FP64 14 x 28 against
+// 12 x 30: C192 69 / 84 us (two full waves / three).
 constexpr int ONE_BAND = 64;
 
 template <class T, int XL, int TH>

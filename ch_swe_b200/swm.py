@@ -179,13 +179,19 @@ class Domain:
                            for t, o in ((17, 3), (17, 4), (25, 2), (25, 3), (25, 4), (33, 2), (33, 3)))
     # the fused stage (linear operator, Ch, SBP 4-2): (maximal tile rows, blocks per SM, 2)
     FUSED_CONFIGS = {"fp32": ((17, 4, 2), (25, 3, 2), (33, 2, 2)), "fp64": ((17, 2, 2), (25, 1, 2))}
+    # the vector stage (Ch, SBP 4-2), per operator and precision
+    VECTOR_CONFIGS = {("linear", "fp32"): ((17, 2, 3), (25, 2, 3), (33, 2, 3)),
+                      ("linear", "fp64"): ((17, 1, 3), (25, 1, 3), (33, 1, 3)),
+                      ("advective", "fp32"): ((25, 2, 3), (33, 2, 3)),
+                      ("advective", "fp64"): ((17, 2, 3), (25, 2, 3), (33, 1, 3))}
 
     @property
     def kernel_config(self) -> tuple:
         """(tile edge, resident blocks per SM, runs) of the stage kernels; runs 1: each
         thread evaluates runs of consecutive outputs along a stencil; runs 2: the fused
         stage (contravariant components computed in the stage kernel, TMA-loaded tiles of
-        at most 26 columns and `tile` rows)."""
+        at most 26 columns and `tile` rows); runs 3: the vector stage (one launch per RK
+        stage of the linear operator, six of the advective one; the default)."""
         t, o, r = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(_lib.load().swe_get_kernel_config(self.ctx, ctypes.byref(t), ctypes.byref(o), ctypes.byref(r)),
               self.ctx, "swe_get_kernel_config")

@@ -270,7 +270,8 @@ int swe_kernel_times(swe_ctx *ctx, swe_stvec *v0, double dt, int nreps, double *
 
 /* Tile size of the stage kernels: the maximal tile edge, 17, 25 or 33 points
    (ceil(N / (tile - 1)) balanced tiles per panel direction).  Contexts start at 25
-   for N <= 96 and 33 above.  No reference counterpart: the reference's tiles are
+   for N <= 96 and 33 above (the split kernels' tile; Ch contexts in SBP 4-2 run the
+   vector stage until a tile or configuration is set).  No reference counterpart: the reference's tiles are
    MPI partitions of the panels (src/parallel/partition_mod.f90:83-129). */
 int swe_set_tile(swe_ctx *ctx, int tile);
 int swe_get_tile(const swe_ctx *ctx, int *tile);
@@ -280,7 +281,12 @@ int swe_get_tile(const swe_ctx *ctx, int *tile);
    Built (tile, blocks) pairs: (17, 3), (17, 4), (25, 2), (25, 3), (25, 4), (33, 2),
    (33, 3), each with runs 0 and 1; swe_set_tile picks (17, 3, 0), (25, 2, 0) or
    (33, 2, 0).  The advective operator's stage kernel always uses the tile's first
-   blocks-per-SM value.  No reference counterpart. */
+   blocks-per-SM value.  runs 2: the fused stage (linear operator, Ch, SBP 4-2).  runs 3:
+   the vector stage of Ch contexts in SBP 4-2, the default from 16 cells on -- linear
+   operator one launch per RK stage, advective six; tile is at least the rows of its
+   tiles.  Linear FP32 (17, 2), (25, 2), (33, 2), FP64 (17, 1), (25, 1), (33, 1);
+   advective FP32 (25, 2), (33, 2), FP64 (17, 2), (25, 2), (33, 1); a configuration that
+   the cube's tiles do not suit returns SWE_EINVAL.  No reference counterpart. */
 int swe_set_kernel_config(swe_ctx *ctx, int tile, int blocks_per_sm, int runs);
 int swe_get_kernel_config(const swe_ctx *ctx, int *tile, int *blocks_per_sm, int *runs);
 /* Autotuner: times nreps graph-replayed RK4 steps of a scratch state for each built
