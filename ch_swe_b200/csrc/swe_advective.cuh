@@ -5,14 +5,14 @@
 //   A  = -(v . grad) u (up4) + Christoffel terms, synchronised on the duplicated
 //        panel-edge points                                     (vector_advection_Ch_mod.f90:33-115)
 // Per RK stage, after k_co2contra (ut, vt and their edge strips):
-//   k_havg   average h over the duplicated panel-edge vertices (in place, as the
-//            reference's ECS_xy halo does to the operator's input)
+//   k_advhalo  average h over the duplicated panel-edge vertices (in place, as the
+//            reference's ECS_xy halo does to the operator's input); covariant u, v at
+//            the virtual points beyond the panel edges (bicubic from the neighbour
+//            face, projected on this face's basis)
 //   k_flux   the up4 mass flux on u and v points, with the virtual h points beyond
 //            the panel edges interpolated along the neighbour's grid lines; also the
 //            flux edge strips for the divergence sync
 //   k_edge   (swe_kernels.cuh) Coriolis from the ut/vt strips, divergence from the flux strips
-//   k_vhalo  covariant u, v at the virtual points beyond the panel edges (bicubic
-//            from the neighbour face, projected on this face's basis)
 //   k_advt   up4 advection and Christoffel terms of u and v, with ut, vt interpolated
 //            to the xy points and back inside its shared-memory tiles
 //   k_stage  (swe_tiled.cuh) divergence of the flux, gradient, Coriolis, A and the RK update
@@ -65,32 +65,28 @@ __device__ __forceinline__ int64_t hb_index(int N, int mem, int t, int s, int a)
 }
 
 // ---------------------------------------------------------------------------
-// k_havg: the averaging of duplicated vertices that the ECS_xy halo procedure
+// havg_block (k_advhalo): the averaging of duplicated vertices that the ECS_xy halo procedure
 // performs on its field (ecs_halo_xy_mod.f90:109-175): corners become the mean of
 // their three copies (in each panel's own order), other edge vertices the mean of
 // their two copies.  The values before the averaging go to HB: the reference's
 // gradient reads its copy h_total taken before (operator_adv_swm_mod.f90:77).
-// Grid (1 + edge blocks, members): block 0 of a member takes the 24 corners (all
-// corner reads precede its corner writes), the others one vertex pair each per
-// thread (edge pairs never touch a corner).
+// Block 0 of a member takes the 24 corners (all corner reads precede its corner
+// writes), the others one vertex pair each per thread (edge pairs never touch a corner).
 // ---------------------------------------------------------------------------
 constexpr int HAVG_THREADS = 256;
 
+__host__ __device__ inline int havg_blocks(int N) { return 1 + (12 * (N - 1) + HAVG_THREADS - 1) / HAVG_THREADS; }
+
 template <class T>
-__global__ void __launch_bounds__(HAVG_THREADS) k_havg(T *__restrict__ Y, T *__restrict__ HB, Dims d,
-                                                       const double *__restrict__ dtm)
+__device__ __forceinline__ void havg_block(T *Y, T *__restrict__ HB, const Dims &d, int mem, int blk)
 {
-    const int mem = blockIdx.y;
-    if (member_frozen(dtm, mem)) return;
-    pdl_trigger();
-    pdl_wait();
     const int N = d.N, n = N + 1;
     T *h = Y + mem * d.ms;   // field 0
     auto at = [&](int t, int i, int j) -> T & { return h[t * d.ps + (j - 1 + MG) * d.P + (i - 1 + MG)]; };
     __shared__ T cval[NPAN * 4];
     const int q = threadIdx.x;
-    if (blockIdx.x > 0) {
-        const int e = (blockIdx.x - 1) * HAVG_THREADS + q;
+    if (blk > 0) {
+        const int e = (blk - 1) * HAVG_THREADS + q;
         if (e >= 12 * (N - 1)) return;
         const int ce = e / (N - 1), a = 2 + e % (N - 1);
         const int t = c_cube_edge[ce][0], s = c_cube_edge[ce][1];
@@ -135,7 +131,7 @@ __global__ void __launch_bounds__(HAVG_THREADS) k_havg(T *__restrict__ Y, T *__r
 // h at xy index (i, j) of panel t, where at most one index lies up to two points
 // beyond the panel: the virtual point is interpolated along the neighbour's grid
 // line at that depth (ecs_halo_xy_mod.f90:177-235); the line's end points are the
-// averaged edge vertices k_havg left in the field.
+// averaged edge vertices k_advhalo left in the field.
 template <class T>
 __device__ __forceinline__ T h_ext(const T *h, const Dims &d, const AdvView<T> &av, int t, int i, int j)
 {
@@ -221,21 +217,14 @@ __global__ void __launch_bounds__(256) k_flux(const T *__restrict__ Y, const T *
 }
 
 // ---------------------------------------------------------------------------
-// k_vhalo: covariant wind at the virtual points beyond the panel edges
+// vhalo_point (k_advhalo): covariant wind at the virtual points beyond the panel edges
 // (ecs_halo_vec_Ch_mod.f90:29-60): bicubic interpolation of the source face's u (y
 // mesh) and v (x mesh), projected on this face's basis vector.
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void __launch_bounds__(256) k_vhalo(const T *__restrict__ Y, T *__restrict__ VH, Dims d, AdvView<T> av,
-                                               int n_members, const double *__restrict__ dtm)
+__device__ __forceinline__ void vhalo_point(const T *Y, T *__restrict__ VH, const Dims &d, const AdvView<T> &av, int mem, int k)
 {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int per = NPAN * av.hp;
-    pdl_trigger();
-    pdl_wait();
-    if (g >= (int64_t)per * n_members) return;
-    const int mem = (int)(g / per), k = (int)(g % per);
-    if (member_frozen(dtm, mem)) return;
     const int p = __ldg(av.hsrc + k);
     const int *ix = av.hidx + 4 * k;
     const T *w = av.hw + 18 * k;
@@ -255,6 +244,33 @@ __global__ void __launch_bounds__(256) k_vhalo(const T *__restrict__ Y, T *__res
     const T vu = bicubic(U, __ldg(ix), __ldg(ix + 1), w, w + 4);
     const T vv = bicubic(V, __ldg(ix + 2), __ldg(ix + 3), w + 8, w + 12);
     VH[(int64_t)mem * per + k] = __ldg(w + 16) * vu + __ldg(w + 17) * vv;
+}
+
+// ---------------------------------------------------------------------------
+// k_advhalo: both of the above in one launch.  The averaging touches h, the wind halo
+// reads u and v, so neither needs the other's result; each is a few microseconds of
+// latency on a handful of blocks.  The first havg_blocks(N) * members blocks average
+// (the corner blocks are the longest chain), the others take one virtual point per thread.
+// Against a launch each (4.5 and 7.3 us at C384 FP32, cold): C96 FP64 65 -> 58 us per RK4
+// step, C384 FP32 178 -> 176 us; ensembles of C48 the same within the runs' spread.
+// ---------------------------------------------------------------------------
+template <class T>
+__global__ void __launch_bounds__(HAVG_THREADS) k_advhalo(T *Y, T *__restrict__ HB, T *__restrict__ VH, Dims d, AdvView<T> av,
+                                                          int n_members, const double *__restrict__ dtm)
+{
+    const int hb = havg_blocks(d.N), b = blockIdx.x;
+    pdl_trigger();
+    pdl_wait();
+    if (b < hb * n_members) {
+        const int mem = b / hb;
+        if (!member_frozen(dtm, mem)) havg_block<T>(Y, HB, d, mem, b % hb);
+        return;
+    }
+    const int64_t g = (int64_t)(b - hb * n_members) * HAVG_THREADS + threadIdx.x;
+    const int per = NPAN * av.hp;
+    if (g >= (int64_t)per * n_members) return;
+    const int mem = (int)(g / per);
+    if (!member_frozen(dtm, mem)) vhalo_point<T>(Y, VH, d, av, mem, (int)(g % per));
 }
 
 // u (y mesh) / v (x mesh) of panel t at an index at most three points beyond the panel

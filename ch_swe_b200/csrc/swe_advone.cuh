@@ -8,7 +8,7 @@
 //               the RK4 update (operator_adv_swm_mod.f90:62-96, rk4_mod.f90:28-40)
 // A tile of k_adv_stage that touches a panel edge reads the neighbour panel's contravariant
 // components and flux beside the edge itself, so the stage needs no edge strips and no
-// edge-sync launch; k_havg and k_vhalo (swe_advective.cuh) stay as they are.
+// edge-sync launch; k_advhalo (swe_advective.cuh) is shared with the split stage.
 //
 // Measured at C384 FP32 per launch (B200, cold L2, ncu): k_co2contra 22.8 -> k_adv_co2 10.6 us,
 // k_stage 55.2 -> k_adv_stage 27 us, k_advt 27.8 -> k_adv_tend 17.8 us, k_edge 6.0 us and its

@@ -1685,12 +1685,10 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
         !encode_rows(&tmW, c->w, sizeof(T), c->dims.P, nrows, bw, bh) || !encode_rows(&tmF, c->fl, sizeof(T), c->dims.P, nrows, bw, bh))
         return false;
     const OneMetric<T> om = one_metric<T>(c, mv);
-    const dim3 hg(1 + (12 * (N - 1) + HAVG_THREADS - 1) / HAVG_THREADS, M);
-    const dim3 vg((unsigned)(((long long)NPAN * av.hp * M + 255) / 256));
+    const dim3 ag((unsigned)(havg_blocks(N) * M + ((long long)NPAN * av.hp * M + HAVG_THREADS - 1) / HAVG_THREADS));
     cudaStream_t st = c->stream, sd = fork ? c->side : c->stream;
     auto co2 = [&] { AdvOneTU<T>::co2(c->olabel, c->oocc, M, tmY, (T *)c->w, c->dims, om, (const T *)c->fmet, dtm, c->derr, st); };
-    auto havg = [&] { launch_k(k_havg<T>, hg, dim3(HAVG_THREADS), 0, sd, (T *)yin, (T *)c->hb, c->dims, dtm); };
-    auto vhalo = [&] { launch_k(k_vhalo<T>, vg, dim3(256), 0, sd, (const T *)yin, (T *)c->vh, c->dims, av, M, dtm); };
+    auto halo = [&] { launch_k(k_advhalo<T>, ag, dim3(HAVG_THREADS), 0, sd, (T *)yin, (T *)c->hb, (T *)c->vh, c->dims, av, M, dtm); };
     auto tend = [&] {
         if (!AdvOneTU<T>::tend(c->olabel, c->oocc, M, tmY, tmW, (const T *)c->vh, (T *)c->adt, c->dims, av, om, mv.inv_hxa, dtm,
                                c->derr, sd))
@@ -1701,9 +1699,8 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
         // the averaging of h, the wind halo and the advective tendencies beside co2 and the flux
         cudaEventRecord(c->ev_fork, st);
         cudaStreamWaitEvent(sd, c->ev_fork, 0);
-        havg();
+        halo();
         cudaEventRecord(c->ev_havg, sd);
-        vhalo();
         co2();
         cudaEventRecord(c->ev_co2, st);
         cudaStreamWaitEvent(sd, c->ev_co2, 0);
@@ -1714,15 +1711,14 @@ static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, voi
         cudaStreamWaitEvent(st, c->ev_side, 0);
     } else {
         co2();
-        havg();
-        vhalo();
+        halo();
         tend();
         flux();
     }
     StageArgs a{mode, dt, c->ones, dtm, c->fl, c->adt, c->hb, c->hs};
     AdvOneTU<T>::stage(c->olabel, c->oocc, M, tmY, tmW, tmF, c->tm_one, (const T *)c->w, (T *)v0, (T *)y1, (T *)acc, (T *)cmp,
                        c->dims, om, a, c->derr, st);
-    c->launches += 6;
+    c->launches += 5;
     return true;
 }
 
@@ -1770,9 +1766,7 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
     const AdvView<T> &av = adv_view<T>(c);
     const int N = c->cfg.N, n = N + 1;
     const dim3 pb(32, 8), pg((n + 31) / 32, (n + 7) / 8, NPAN * M);
-    const dim3 hg(1 + (12 * (N - 1) + HAVG_THREADS - 1) / HAVG_THREADS, M);
-    const long long nvh = (long long)NPAN * av.hp * M;
-    const dim3 vg((unsigned)((nvh + 255) / 256));
+    const dim3 ag((unsigned)(havg_blocks(N) * M + ((long long)NPAN * av.hp * M + HAVG_THREADS - 1) / HAVG_THREADS));
     const bool fork = c->side && c->branches;
     if (c->one) {
         if (enqueue_adv_one<T>(c, yin, v0, y1, acc, cmp, mode, dt, dtm, mv, fork)) return;
@@ -1786,9 +1780,8 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
         // k_co2contra, k_flux and k_edge, and join before the stage kernel.
         cudaEventRecord(c->ev_fork, c->stream);
         cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-        launch_k(k_havg<T>, hg, dim3(HAVG_THREADS), 0, c->side, (T *)yin, (T *)c->hb, c->dims, dtm);
+        launch_k(k_advhalo<T>, ag, dim3(HAVG_THREADS), 0, c->side, (T *)yin, (T *)c->hb, (T *)c->vh, c->dims, av, M, dtm);
         cudaEventRecord(c->ev_havg, c->side);
-        launch_k(k_vhalo<T>, vg, dim3(256), 0, c->side, (const T *)yin, (T *)c->vh, c->dims, av, M, dtm);
         if (!launch_co2contra<T>(c->tile, c->occ, c->runs, c->ord, M, (const T *)yin, (T *)c->w, (T *)c->es, c->dims, mv,
                             c->stream, dtm)) c->launch_miss = true;
         cudaEventRecord(c->ev_co2, c->stream);
@@ -1799,7 +1792,7 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
     } else {
         if (!launch_co2contra<T>(c->tile, c->occ, c->runs, c->ord, M, (const T *)yin, (T *)c->w, (T *)c->es, c->dims, mv,
                             c->stream, dtm)) c->launch_miss = true;
-        launch_k(k_havg<T>, hg, dim3(HAVG_THREADS), 0, c->stream, (T *)yin, (T *)c->hb, c->dims, dtm);
+        launch_k(k_advhalo<T>, ag, dim3(HAVG_THREADS), 0, c->stream, (T *)yin, (T *)c->hb, (T *)c->vh, c->dims, av, M, dtm);
     }
     launch_k(k_flux<T>, pg, pb, 0, c->stream, (const T *)yin, (const T *)c->w, (T *)c->fl, (T *)c->fs, c->dims, av, dtm,
              ord_strip_lines(c->ord));
@@ -1808,13 +1801,12 @@ static void enqueue_stage(swe_ctx *c, const void *yin, void *v0, void *y1, void 
     if (fork) {
         cudaStreamWaitEvent(c->stream, c->ev_side, 0);
     } else {
-        launch_k(k_vhalo<T>, vg, dim3(256), 0, c->stream, (const T *)yin, (T *)c->vh, c->dims, av, M, dtm);
         launch_adv<T>(c, yin, av, mv, dtm, c->stream);
     }
     StageArgs a{mode, dt, c->ones, dtm, c->fl, c->adt, c->hb, c->hs};
     if (!launch_stage<T>(c->tile, c->occ, c->runs, c->ord, M, (const T *)yin, (const T *)c->w, (const T *)c->edge, (T *)v0, (T *)y1, (T *)acc,
                     (T *)cmp, c->dims, mv, a, c->stream)) c->launch_miss = true;
-    c->launches += 7;
+    c->launches += 6;
 }
 
 static void enqueue_apply(swe_ctx *c, void *out, const void *in)

@@ -149,3 +149,31 @@ def test_advective_apply_matches_oracle(precision, cfg, N, orography):
     for g, r, name in zip(y.download(), ref, "huv"):
         assert rel(g, r) < RTOL[precision], (name, rel(g, r))
     dom.destroy()
+
+
+@pytest.mark.parametrize("cfg", [(25, 2, 0), (25, 2, 3)])
+@pytest.mark.parametrize("N", [22, 23])
+def test_advective_members_share_the_halo_launch(N, cfg):
+    """Edge averages and virtual winds of all members in one launch: 252 edge vertices fit one
+    block of a member, 264 need two; member 1 is frozen."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    from oracle.oracle import Oracle
+    M = 3
+    states = [random_state(N, 600 + 10 * N + k) for k in range(M)]
+    stack = [np.stack([s[f] + (0.0 if f else 1000.0) for s in states]) for f in range(3)]
+    dts = np.array([60.0, 0.0, 30.0])
+    dom = create_domain(N, n_members=M, operator="advective")
+    dom.kernel_config = cfg
+    op = create_swm_operator(dom.grav, {"swm_operator_type": "advective_swm_operator"}, dom)
+    st = create_stvec_swm(dom).upload(*stack, member=None)
+    create_timescheme(st, "rk4").steps_members(st, op, dts, 2)
+    dom.synchronize()
+    out = st.download(member=None)
+    o = Oracle(N, operator="advective")
+    for m in (0, 2):
+        ref = o.rk4(*(f[m] for f in stack), dts[m], 2)
+        for g, r, name in zip(out, ref, "huv"):
+            assert rel(g[m], r) < 1e-12, (m, name, rel(g[m], r))
+    for f in range(3):
+        assert np.array_equal(out[f][1], stack[f][1])
+    dom.destroy()
