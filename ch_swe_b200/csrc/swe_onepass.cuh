@@ -91,9 +91,20 @@ enum { OB_TF = 0, OB_NQ = 5, OB_JT = 6, OB_T = 7 };
 
 // Named barriers: the main threads' passes; main to band (J ut, J vt are there); band to
 // main (the boundary vertices are there); all band threads (corners); one per side.
+// bar.sync and bar.arrive are the aligned forms: every thread of the warp has to execute the
+// same one together, so the warp reconverges first (the barriers follow divergent branches:
+// thread 0's tile loads, the band threads' boundary and corner points).
 enum { BAR_MAIN = 1, BAR_P2 = 2, BAR_BND = 3, BAR_CORN = 4, BAR_SIDE = 5 };
-__device__ __forceinline__ void nbar_sync(int id, int cnt) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory"); }
-__device__ __forceinline__ void nbar_arrive(int id, int cnt) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(cnt) : "memory"); }
+__device__ __forceinline__ void nbar_sync(int id, int cnt)
+{
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory");
+}
+__device__ __forceinline__ void nbar_arrive(int id, int cnt)
+{
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(cnt) : "memory");
+}
 
 // The inputs of VW consecutive outputs of an interior x row: c2i own-2 .. own+VW (SH = -2),
 // i2c own-1 .. own+VW+1 (SH = -1).
