@@ -348,6 +348,21 @@ static int fail(swe_ctx *c, int code, const char *fmt, ...)
         CU(ctx, cudaGetLastError());                                                                            \
     } while (0)
 
+// Copies to and clears of device memory, complete on return.  They go through the context's
+// stream: it does not wait for the default stream, where a copy from pageable memory returns
+// before it has landed and a clear before it has run -- behind whatever the host program has
+// queued there.
+static cudaError_t to_device(swe_ctx *c, void *dst, const void *src, size_t bytes, cudaMemcpyKind kind = cudaMemcpyHostToDevice)
+{
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, c->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+static cudaError_t clear_device(swe_ctx *c, void *p, size_t bytes)
+{
+    cudaError_t e = cudaMemsetAsync(p, 0, bytes, c->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
 static bool g_tables_ready[64] = {false};
 
 // Maximal tile sizes the stage kernels are built for; ceil(N / (TM - 1)) balanced
@@ -412,7 +427,8 @@ static cudaError_t upload_link_tables()
     if (e == cudaSuccess) e = AdvOneTU<double>::upload_tables(l);
     if (e == cudaSuccess) e = GroupTU<float>::upload_tables(l, q);
     if (e == cudaSuccess) e = GroupTU<double>::upload_tables(l, q);
-    return e;
+    // the kernels that read them run on streams that do not wait for the default stream's copies
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
 static int upload_tables(swe_ctx *c)
@@ -475,7 +491,7 @@ static int build_metric(swe_ctx *c, DevMetric<T> &dm)
     T *d = nullptr;
     if (cudaMalloc(&d, n_el * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "metric allocation failed");
     dm.base = d;
-    CU(c, cudaMemcpy(d, h.data(), n_el * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, d, h.data(), n_el * sizeof(T)));
     MetricView<T> &v = dm.v;
     v.Q11y = d; v.iJy = d + box; v.Jy = d + 2 * box; v.Q22x = d + 3 * box; v.iJx = d + 4 * box; v.Jx = d + 5 * box;
     v.JQ12 = d + 6 * box; v.iJa = d + 7 * box; v.fJ2 = d + 8 * box;
@@ -487,7 +503,6 @@ static int build_metric(swe_ctx *c, DevMetric<T> &dm)
     v.inv_hxa = T(1.0 / (hx * a));
     v.inv_hx = T(1.0 / hx);
     v.grav = T(c->cfg.grav);
-    CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // the copy above, before the kernel on the context's stream
     k_edge_tables<T><<<(N + 1 + 127) / 128, 128, 0, c->stream>>>(v, c->dims, ej, ef, ea, ord_strip_lines(c->ord));
     CU(c, cudaGetLastError());
     CU(c, cudaStreamSynchronize(c->stream));
@@ -562,10 +577,9 @@ static int build_fused_metric(swe_ctx *c, const MetricView<T> &mv)
     T *d = nullptr;
     if (cudaMalloc(&d, h.size() * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "fused metric allocation failed");
     c->fmet = d;
-    CU(c, cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, d, h.data(), h.size() * sizeof(T)));
     // f J^2 per panel: the same values the split kernels use
-    CU(c, cudaMemcpy(d + FM_FJ2 * box, mv.fJ2, NPAN * box * sizeof(T), cudaMemcpyDeviceToDevice));
-    CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // before kernels on the context's stream
+    CU(c, to_device(c, d + FM_FJ2 * box, mv.fJ2, NPAN * box * sizeof(T), cudaMemcpyDeviceToDevice));
     return SWE_OK;
 }
 
@@ -628,8 +642,7 @@ static int build_one_tables(swe_ctx *c)
     T *d = nullptr;
     if (cudaMalloc(&d, (Z::SIDE + ns) * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "stage table allocation failed");
     c->onetab = d;
-    CU(c, cudaMemcpy(d, wt.data(), wt.size() * sizeof(T), cudaMemcpyHostToDevice));
-    CU(c, cudaStreamSynchronize(cudaStreamLegacy));
+    CU(c, to_device(c, d, wt.data(), wt.size() * sizeof(T)));
     OneTU<T>::tables((const T *)c->fmet, d + Z::SIDE, c->dims, c->stream);
     CU(c, cudaGetLastError());
     CU(c, cudaStreamSynchronize(c->stream));
@@ -707,7 +720,7 @@ static int build_c_metric(swe_ctx *c)
     T *d = nullptr;
     if (cudaMalloc(&d, h.size() * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "C metric allocation failed");
     c->cmet = d;
-    CU(c, cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, d, h.data(), h.size() * sizeof(T)));
     return SWE_OK;
 }
 
@@ -764,10 +777,10 @@ static int build_ah_metric(swe_ctx *c, DevAh<T> &da)
     T *d = nullptr;
     if (cudaMalloc(&d, h.size() * sizeof(T)) != cudaSuccess) return fail(c, SWE_ENOMEM, "Ah metric allocation failed");
     da.base = d;
-    CU(c, cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, d, h.data(), h.size() * sizeof(T)));
     da.v.J = d; da.v.Q1 = d + box; da.v.Q2 = d + 2 * box; da.v.Q3 = d + 3 * box; da.v.fJ = d + 4 * box;
     if (cudaMalloc(&c->qa, box * sizeof(double)) != cudaSuccess) return fail(c, SWE_ENOMEM, "Ah quadrature allocation failed");
-    CU(c, cudaMemcpy(c->qa, q.data(), box * sizeof(double), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, c->qa, q.data(), box * sizeof(double)));
     return SWE_OK;
 }
 
@@ -969,8 +982,8 @@ static int build_adv_tables(swe_ctx *c, DevAdv<T> &da)
         }
     if (cudaMalloc(&da.base, n_el * sizeof(T)) != cudaSuccess || cudaMalloc(&da.ibase, n_int * sizeof(int)) != cudaSuccess)
         return fail(c, SWE_ENOMEM, "advective tables allocation failed");
-    CU(c, cudaMemcpy(da.base, h.data(), n_el * sizeof(T), cudaMemcpyHostToDevice));
-    CU(c, cudaMemcpy(da.ibase, hi.data(), n_int * sizeof(int), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, da.base, h.data(), n_el * sizeof(T)));
+    CU(c, to_device(c, da.ibase, hi.data(), n_int * sizeof(int)));
     AdvView<T> &v = da.v;
     v.xyw = da.base;
     v.hw = da.base + o_hw;
@@ -1030,7 +1043,7 @@ static int build_quadrature(swe_ctx *c)
     }
     if (cudaMalloc(&c->qw, h.size() * sizeof(double)) != cudaSuccess)
         return fail(c, SWE_ENOMEM, "quadrature allocation failed");
-    CU(c, cudaMemcpy(c->qw, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, c->qw, h.data(), h.size() * sizeof(double)));
     if (cudaMalloc(&c->red, 4096 * sizeof(double)) != cudaSuccess)
         return fail(c, SWE_ENOMEM, "reduction buffer allocation failed");
     return SWE_OK;
@@ -1089,10 +1102,7 @@ static int alloc_box(swe_ctx *c, void **p)
 {
     size_t bytes = c->box_elems * c->elem;
     if (cudaMalloc(p, bytes) != cudaSuccess) return fail(c, SWE_ENOMEM, "device allocation of %zu bytes failed", bytes);
-    CU(c, cudaMemset(*p, 0, bytes));
-    // the context's stream does not block on the default stream: without this wait the clear
-    // could run after an upload there and wipe the uploaded state
-    CU(c, cudaStreamSynchronize(cudaStreamLegacy));
+    CU(c, clear_device(c, *p, bytes));
     return SWE_OK;
 }
 
@@ -1188,8 +1198,8 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
     if (cudaMalloc(&c->Hm, sizeof(double) * cfg->n_members) != cudaSuccess) return bail(SWE_ENOMEM);
     if (cudaMalloc(&c->dtm, sizeof(double) * cfg->n_members) != cudaSuccess) return bail(SWE_ENOMEM);
     if (cudaMalloc(&c->derr, sizeof(int)) != cudaSuccess) return bail(SWE_ENOMEM);
-    if (cudaMemset(c->derr, 0, sizeof(int)) != cudaSuccess) return bail(SWE_ECUDA);
-    if (cudaMemcpy(c->Hm, c->Hhost.data(), sizeof(double) * cfg->n_members, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (clear_device(c, c->derr, sizeof(int)) != cudaSuccess) return bail(SWE_ECUDA);
+    if (to_device(c, c->Hm, c->Hhost.data(), sizeof(double) * cfg->n_members) != cudaSuccess)
         return bail(SWE_ECUDA);
     if ((rc = alloc_box(c, &c->ya)) || (rc = alloc_box(c, &c->yb)) || (rc = alloc_box(c, &c->acc)) ||
         (rc = alloc_box(c, &c->w)))
@@ -1197,24 +1207,24 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
     {
         const size_t eb = (size_t)cfg->n_members * NPAN * 4 * (N + 1) * 3 * c->elem;
         if (cudaMalloc(&c->edge, eb) != cudaSuccess) return bail(SWE_ENOMEM);
-        if (cudaMemset(c->edge, 0, eb) != cudaSuccess) return bail(SWE_ECUDA);
+        if (clear_device(c, c->edge, eb) != cudaSuccess) return bail(SWE_ECUDA);
         const size_t sb = (size_t)strip_member(N, cfg->n_members, ord_strip_lines(ord)) * c->elem;
         if (cudaMalloc(&c->es, sb) != cudaSuccess) return bail(SWE_ENOMEM);
-        if (cudaMemset(c->es, 0, sb) != cudaSuccess) return bail(SWE_ECUDA);
+        if (clear_device(c, c->es, sb) != cudaSuccess) return bail(SWE_ECUDA);
         if (cfg->operator_kind == SWE_OP_ADVECTIVE) {
             c->adv = true;
             if ((rc = alloc_box(c, &c->fl)) || (rc = alloc_box(c, &c->adt))) return bail(rc);
             if (cudaMalloc(&c->fs, sb) != cudaSuccess) return bail(SWE_ENOMEM);
-            if (cudaMemset(c->fs, 0, sb) != cudaSuccess) return bail(SWE_ECUDA);
+            if (clear_device(c, c->fs, sb) != cudaSuccess) return bail(SWE_ECUDA);
             const size_t vb = (size_t)cfg->n_members * NPAN * vh_points(N) * c->elem;
             if (cudaMalloc(&c->vh, vb) != cudaSuccess) return bail(SWE_ENOMEM);
-            if (cudaMemset(c->vh, 0, vb) != cudaSuccess) return bail(SWE_ECUDA);
+            if (clear_device(c, c->vh, vb) != cudaSuccess) return bail(SWE_ECUDA);
             const size_t hbb = (size_t)cfg->n_members * NPAN * 4 * (N + 1) * c->elem;
             if (cudaMalloc(&c->hb, hbb) != cudaSuccess) return bail(SWE_ENOMEM);
-            if (cudaMemset(c->hb, 0, hbb) != cudaSuccess) return bail(SWE_ECUDA);
+            if (clear_device(c, c->hb, hbb) != cudaSuccess) return bail(SWE_ECUDA);
             std::vector<double> one(cfg->n_members, 1.0);
             if (cudaMalloc(&c->ones, sizeof(double) * cfg->n_members) != cudaSuccess) return bail(SWE_ENOMEM);
-            if (cudaMemcpy(c->ones, one.data(), sizeof(double) * cfg->n_members, cudaMemcpyHostToDevice) != cudaSuccess)
+            if (to_device(c, c->ones, one.data(), sizeof(double) * cfg->n_members) != cudaSuccess)
                 return bail(SWE_ECUDA);
             rc = cfg->precision == SWE_FP64 ? build_adv_tables<double>(c, c->a64) : build_adv_tables<float>(c, c->a32);
             if (rc != SWE_OK) return bail(rc);
@@ -1235,9 +1245,6 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
     if (cudaHostAlloc((void **)&c->pinned, c->box_elems * c->elem, cudaHostAllocDefault) != cudaSuccess)
         return bail(SWE_ENOMEM);
     std::memset(c->pinned, 0, c->box_elems * c->elem);
-    // every table and cleared buffer in place, whatever stream the context works on next
-    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
-        return bail(SWE_ECUDA);
     *out = c;
     return SWE_OK;
 }
@@ -1270,7 +1277,7 @@ extern "C" int swe_synchronize(swe_ctx *c)
     int flag = 0;
     CU(c, cudaMemcpy(&flag, c->derr, sizeof(int), cudaMemcpyDeviceToHost));
     if (flag) {
-        CU(c, cudaMemset(c->derr, 0, sizeof(int)));
+        CU(c, clear_device(c, c->derr, sizeof(int)));
         return fail(c, SWE_ECUDA, "a stage kernel gave up waiting for its tile loads; its outputs are incomplete");
     }
     return SWE_OK;
@@ -2394,8 +2401,7 @@ static int dif_setup(swe_ctx *c)
                 }
         if (cudaMalloc(&c->dif_b, h.size() * sizeof(T)) != cudaSuccess)
             return fail(c, SWE_ENOMEM, "diffusion basis allocation failed");
-        CU(c, cudaMemcpy(c->dif_b, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-        CU(c, cudaStreamSynchronize(cudaStreamLegacy));   // before kernels on the context's stream
+        CU(c, to_device(c, c->dif_b, h.data(), h.size() * sizeof(T)));
     }
     if (!c->dif && cudaMalloc(&c->dif, 5 * M * DIF_FIELDS * NPAN * box * sizeof(T)) != cudaSuccess)
         return fail(c, SWE_ENOMEM, "diffusion scratch allocation failed");
@@ -2780,7 +2786,7 @@ static int ensure_otab(swe_ctx *c)
         c->otab = nullptr;
         return fail(c, SWE_ENOMEM, "diagnostic table allocation failed");
     }
-    CU(c, cudaMemcpy(c->otab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, c->otab, h.data(), h.size() * sizeof(double)));
     return SWE_OK;
 }
 
@@ -3176,8 +3182,8 @@ static int ensure_latlon(swe_ctx *c, int nlat, int nlon)
         cudaFree(c->ll_i); c->ll_i = nullptr; c->ll_d = nullptr;
         return fail(c, SWE_ENOMEM, "lat-lon regrid allocation failed");
     }
-    CU(c, cudaMemcpy(c->ll_i, hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CU(c, cudaMemcpy(c->ll_d, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, c->ll_i, hi.data(), hi.size() * sizeof(int)));
+    CU(c, to_device(c, c->ll_d, hd.data(), hd.size() * sizeof(double)));
     c->ll_nlat = nlat;
     c->ll_nlon = nlon;
     return SWE_OK;
@@ -3396,8 +3402,8 @@ static int ensure_latlon_o(swe_ctx *c, int nlat, int nlon)
         cudaFree(c->llo_i); c->llo_i = nullptr; c->llo_d = nullptr;
         return fail(c, SWE_ENOMEM, "lat-lon curl regrid allocation failed");
     }
-    CU(c, cudaMemcpy(c->llo_i, hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CU(c, cudaMemcpy(c->llo_d, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CU(c, to_device(c, c->llo_i, hi.data(), hi.size() * sizeof(int)));
+    CU(c, to_device(c, c->llo_d, hd.data(), hd.size() * sizeof(double)));
     c->llo_nlat = nlat;
     c->llo_nlon = nlon;
     return SWE_OK;
@@ -3417,7 +3423,7 @@ static int enqueue_div(swe_ctx *c, const void *yin, const MetricView<T> &mv)
             c->negones = nullptr;
             return fail(c, SWE_ENOMEM, "divergence factor allocation failed");
         }
-        CU(c, cudaMemcpy(c->negones, neg.data(), sizeof(double) * M, cudaMemcpyHostToDevice));
+        CU(c, to_device(c, c->negones, neg.data(), sizeof(double) * M));
     }
     if (!launch_co2contra<T>(c->tile, c->occ, c->runs, c->ord, M, (const T *)yin, (T *)c->w, (T *)c->es, c->dims, mv,
                         c->stream, nullptr)) c->launch_miss = true;

@@ -2,8 +2,9 @@
 
 A context's stream does not wait for the default stream, where a host program may have
 kernels of its own queued (torch's current stream is that one).  Buffers cleared or tables
-copied there are late whenever it is busy: here it is kept busy while a context is created and
-its state uploaded and advanced.  Every result has the bits that it has on an idle device.
+copied there are late whenever it is busy: here it is kept busy while a context is created,
+its state uploaded and advanced, and while the diagnostics build their tables on first use.
+Every result has the bits that it has on an idle device.
 """
 import numpy as np
 import pytest
@@ -77,3 +78,27 @@ def test_first_pass_of_a_fresh_context(N, kw):
     if not kw:
         for g, r in zip(out[1][1:], Oracle(N, h_mean=1000.0).rk4(*ic, 10.0, 3)):
             assert np.abs(g - r).max() < 1e-12 * np.abs(r).max()
+
+
+@pytest.mark.parametrize("what", ["curl", "energies", "h", "div", "regrid_curl", "wind"])
+@pytest.mark.parametrize("N", [8, 24])
+def test_tables_of_the_diagnostics_on_first_use(N, what):
+    from ch_swe_b200.diag import LatlonOutputer, LatlonVecOutputer, SwmOutputDiag
+    out = []
+    for wait in (idle, busy):
+        _, dom, _, st = make(N, wait)
+        idle()
+        wait()
+        if what == "curl":
+            r = [SwmOutputDiag(dom).curl(st)]
+        elif what == "energies":
+            r = [np.array(list(SwmOutputDiag(dom).calc_energies(st).values()))]
+        elif what == "wind":
+            r = list(LatlonVecOutputer(dom, 8, 16).regrid(st))
+        else:
+            r = [getattr(LatlonOutputer(dom, 8, 16), {"h": "regrid"}.get(what, what if what.startswith("regrid") else "regrid_" + what))(st)]
+        out.append([np.array(a) for a in r])
+        idle()
+        dom.destroy()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -16,3 +16,15 @@ def test_named_barriers_follow_a_reconvergence():
             assert re.search(r"__syncwarp\(\);\s*$", src[:m.start()]), (os.path.basename(path), src[m.start():m.start() + 60])
             seen += 1
     assert seen >= 2
+
+
+def test_no_transfer_to_the_device_on_the_default_stream():
+    """Contexts work on streams that do not wait for the default stream: what a copy or a clear
+    there leaves in device memory has no order against their kernels."""
+    for path in glob.glob(os.path.join(ROOT, "ch_swe_b200", "csrc", "*.cu*")):
+        src = re.sub(r"//[^\n]*", "", open(path).read())
+        assert not re.search(r"cudaMemset\(|cudaMemcpy\([^;]*(HostToDevice|DeviceToDevice)", src), os.path.basename(path)
+    src = open(os.path.join(ROOT, "ch_swe_b200", "csrc", "swe_api.cu")).read()
+    body = src[src.index("static cudaError_t upload_link_tables()"):]
+    body = body[:body.index("\n}")]
+    assert body.rindex("cudaStreamSynchronize(cudaStreamLegacy)") > body.rindex("upload_tables(")
