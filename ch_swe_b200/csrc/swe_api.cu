@@ -2417,6 +2417,25 @@ static double dif_coeff(const swe_ctx *c, double coeff)
     return -1.0 * ((dc * dc) * (dc * dc));
 }
 
+// The difference passes of one Laplacian: src -> dst inside the panels, R on their boundaries.
+template <class T, int ORD, bool VEC>
+static void launch_laplacian(swe_ctx *c, const DifSplit &sp, const T *src, T *D1X, T *D1Y, T *R, T *dst, const AhView<T> &av,
+                             const DifView<T> &dv)
+{
+    const int co = dif_carveout(c->cfg.N, c->cfg.n_members);
+    const dim3 g(DIF_HALF * (sp.ne + sp.ni), 1, NPAN * c->cfg.n_members * (DIF_FIELDS / DIF_HALF)), b(DIF_NT);
+    launch_carveout(co, k_dif_d1<T, ORD, VEC>, g, b, 0, c->stream, src, D1X, D1Y, c->dims, av, sp);
+    launch_carveout(co, k_dif_lap<T, ORD, VEC>, g, b, 0, c->stream, src, (const T *)D1X, (const T *)D1Y, R, dst, c->dims, av, dv, sp);
+}
+template <class T, int ORD>
+static void launch_laplacian(swe_ctx *c, const T *src, T *D1X, T *D1Y, T *R, T *dst, const AhView<T> &av, const DifView<T> &dv)
+{
+    const DifSplit sp = dif_split<T, ORD>(c->cfg.N, c->cfg.n_members);
+    if constexpr (dif_vectors<T>(ORD))
+        if (sp.nr) return launch_laplacian<T, ORD, true>(c, sp, src, D1X, D1Y, R, dst, av, dv);
+    launch_laplacian<T, ORD, false>(c, sp, src, D1X, D1Y, R, dst, av, dv);
+}
+
 // y: the state (read; updated in place unless out), out: the tendency (apply).
 template <class T>
 static int enqueue_diffusion(swe_ctx *c, T *y, T *out, double dt, const double *dtm, int lap_order, double uv_coeff,
@@ -2424,7 +2443,7 @@ static int enqueue_diffusion(swe_ctx *c, T *y, T *out, double dt, const double *
 {
     int rc = dif_setup<T>(c);
     if (rc) return rc;
-    const int N = c->cfg.N, n = N + 1, M = c->cfg.n_members;
+    const int N = c->cfg.N, n = N + 1, M = c->cfg.n_members, co = dif_carveout(N, M);
     const Dims d = c->dims;
     const size_t set = (size_t)M * DIF_FIELDS * NPAN * d.ps;
     T *X = (T *)c->dif, *D1X = X + set, *D1Y = X + 2 * set, *R = X + 3 * set, *A = X + 4 * set;
@@ -2436,25 +2455,22 @@ static int enqueue_diffusion(swe_ctx *c, T *y, T *out, double dt, const double *
     const DifView<T> dv{(const T *)c->dif_b, mb42, mb63, w21, w42, w63, hxa * hxa};
     const dim3 pb(32, 8), pm((n + 31) / 32, (n + 7) / 8, NPAN * M);
     const dim3 sg((4 * N + 255) / 256, 1, NPAN * M * DIF_FIELDS);
-    launch_k(k_dif_prep<T>, pm, pb, 0, c->stream, (const T *)y, X, d, dv);
+    launch_carveout(co, k_dif_prep<T>, pm, pb, 0, c->stream, (const T *)y, X, d, dv);
     // L(X) -> A, then L(A) -> X
-    const DifSplit sp = dif_split(N, lap_order, OV<T>::W);
-    const dim3 pf(sp.ni + sp.ne, 1, NPAN * M * (DIF_FIELDS / DIF_PAIR));
     T *src = X, *dst = A;
     for (int pass = 0; pass < 2; pass++) {
-        launch_k(lap_order == 63 ? k_dif_d1<T, 63> : (lap_order == 42 ? k_dif_d1<T, 42> : k_dif_d1<T, 21>), pf,
-                 dim3(256), 0, c->stream, (const T *)src, D1X, D1Y, d, av, sp);
-        launch_k(lap_order == 63 ? k_dif_lap<T, 63> : (lap_order == 42 ? k_dif_lap<T, 42> : k_dif_lap<T, 21>), pf,
-                 dim3(256), 0, c->stream, (const T *)src, (const T *)D1X, (const T *)D1Y, R, dst, d, av, dv, sp);
-        launch_k(k_dif_sync<T>, sg, dim3(256), 0, c->stream, (const T *)R, dst, d);
+        if (lap_order == 63) launch_laplacian<T, 63>(c, src, D1X, D1Y, R, dst, av, dv);
+        else if (lap_order == 42) launch_laplacian<T, 42>(c, src, D1X, D1Y, R, dst, av, dv);
+        else launch_laplacian<T, 21>(c, src, D1X, D1Y, R, dst, av, dv);
+        launch_carveout(co, k_dif_sync<T>, sg, dim3(256), 0, c->stream, (const T *)R, dst, d);
         std::swap(src, dst);
     }
-    launch_k(k_dif_vraw<T>, pm, pb, 0, c->stream, (const T *)X, D1X, D1Y, d, dv, T(dif_coeff(c, uv_coeff)));
+    launch_carveout(co, k_dif_vraw<T>, pm, pb, 0, c->stream, (const T *)X, D1X, D1Y, d, dv, T(dif_coeff(c, uv_coeff)));
     if (out)
-        launch_k(k_dif_update<T, true>, pm, pb, 0, c->stream, y, out, (const T *)X, (const T *)D1X, (const T *)D1Y, d, mv,
+        launch_carveout(co, k_dif_update<T, true>, pm, pb, 0, c->stream, y, out, (const T *)X, (const T *)D1X, (const T *)D1Y, d, mv,
                  T(dif_coeff(c, h_coeff)), T(0), (const double *)nullptr);
     else
-        launch_k(k_dif_update<T, false>, pm, pb, 0, c->stream, y, (T *)nullptr, (const T *)X, (const T *)D1X,
+        launch_carveout(co, k_dif_update<T, false>, pm, pb, 0, c->stream, y, (T *)nullptr, (const T *)X, (const T *)D1X,
                  (const T *)D1Y, d, mv, T(dif_coeff(c, h_coeff)), T(dt), dtm);
     c->launches += 9;
     return SWE_OK;

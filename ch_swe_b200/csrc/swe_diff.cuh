@@ -184,41 +184,76 @@ __global__ void __launch_bounds__(256) k_dif_prep(const T *__restrict__ Y, T *__
         X[dif_base(d, mem, 1 + k) + t * d.ps + o] = b[k * d.ps] * u + b[(3 + k) * d.ps] * w;
 }
 
+// Blocks of the difference passes.  One field per thread, 128 threads: blockIdx.x takes the
+// single vertices (the longest chains) of the two fields of blockIdx.z first, then their
+// interior vectors.  With two fields per thread (the metric read once for both) a diffusion
+// step of C124 x 4 took 125 / 211 us (FP32, 4-2 / 6-3; point-wise before that 120 / 140, now
+// 99 / 126): twice the chain in a closure vertex, a quarter of the blocks, and 123 to 170
+// registers in blocks of 256.
+constexpr int DIF_NT = 128, DIF_HALF = 2;
+// Blocks per SM that k_dif_lap's registers leave room for.  Without vectors the kernels are
+// instantiations of their own: few enough registers that the next launch's blocks fit beside
+// them and start early.
+template <class T>
+__host__ __device__ constexpr int dif_minb(int ord, bool vec) { return !vec ? 10 : (sizeof(T) == 4 && ord != 21 ? 8 : 6); }
+// Vertices of all fields from which on the interior goes by vectors (never in FP64 6-3, whose
+// vectors of two points read as many words as they save) and the diffusion's launches ask for
+// little shared memory (dif_carveout).  us per RK4 step with diffusion, alone, vectors / single
+// vertices, in parentheses with the carveout:
+//   C48       2-1 FP32 60.5 / 56.0 (62.9 / 61.9), FP64 63.6 / 61.4 (66.9 / 64.0)
+//             4-2      89.4 / 89.3 (93.7 / 92.7),     104.4 / 99.7 (103.9 / 103.1)
+//   C75       2-1      60.2 / 58.7 (65.0 / 62.0),      65.2 / 64.1 (67.1 / 64.3)
+//             4-2      89.9 / 85.5 (94.6 / 88.5),     100.0 / 98.3 (98.9 / 97.2)
+//   C96       2-1      65.9 / 65.2 (66.6 / 65.6),      74.9 / 71.9 (72.8 / 72.6)
+//             4-2     100.0 / 100.4 (95.6 / 96.8),    119.4 / 118.4 (111.2 / 111.2)
+//   C192      4-2     135.2 / 146.8 (127.3 / 146.5),  183.0 / 188.9 (180.2 / 187.8)
+//   4 x C192  4-2     318 / 400 (316 / 400),          502 / 532 (496 / 531)
+constexpr long long DIF_LARGE = 200000;
+template <class T>
+__host__ __device__ constexpr bool dif_vectors(int ord) { return sizeof(T) == 4 || ord != 63; }
+static inline bool dif_large(int N, int members) { return (long long)(N + 1) * (N + 1) * NPAN * DIF_FIELDS * members >= DIF_LARGE; }
+// Percent of the SM's L1 as shared memory, which the diffusion's kernels do not use: one value
+// for all of its launches, so that no SM drains to change it between them.
+static inline int dif_carveout(int N, int members) { return dif_large(N, members) ? 8 : cudaSharedmemCarveoutDefault; }
+
 // Split of a panel's n x n vertices for the difference passes: the vectors (swe_vec.cuh)
 // whose points and rows all take interior rows of both the narrow second difference and the
 // first difference, and the remaining vertices, one per thread.  The two parts are blocks
-// of their own: a warp never waits for closure rows beside its interior points.
+// of their own: a warp never waits for closure rows beside its interior points.  Without
+// interior vectors (nr == 0) every vertex takes a thread, in blocks of 32 columns.
 struct DifSplit {
-    int n, va, nv, lo, nr;   // first vector, vectors per row, first row, rows; nv * nr == 0: none
-    int ni, ne;              // blocks of the interior vectors and of the other vertices
+    int n, va, nv, lo, nr;   // first vector, vectors per row, first row, rows; nr == 0: none
+    int ne, ni;              // blocks of a field's single vertices and of its interior vectors
 };
 __host__ __device__ constexpr int dif_lo(int ord) { return ord == 21 ? 2 : (ord == 42 ? 7 : 10); }
-static inline DifSplit dif_split(int N, int ord, int VW)
+template <class T, int ORD>
+static inline DifSplit dif_split(int N, int members)
 {
+    constexpr int VW = OV<T>::W, NT = DIF_NT, R = NT / 32;
     DifSplit s{};
-    const int n = N + 1, lo = dif_lo(ord), hi = n + 1 - lo;
+    const int n = N + 1, lo = dif_lo(ORD), hi = n + 1 - lo;
     s.n = n;
     s.lo = lo;
     s.va = (lo - 1 + VW - 1) / VW;
     s.nv = hi / VW - s.va;
     s.nr = hi - lo + 1;
-    if (s.nv < 1 || s.nr < 1) s.nv = s.nr = 0;
-    s.ni = (s.nv * s.nr + 255) / 256;
-    s.ne = (n * n - s.nv * VW * s.nr + 255) / 256;
+    if (!dif_vectors<T>(ORD) || s.nv < 1 || s.nr < 1 || !dif_large(N, members)) s.nv = s.nr = 0;
+    s.ni = (s.nv * s.nr + NT - 1) / NT;
+    s.ne = s.nr ? (n * n - s.nv * VW * s.nr + NT - 1) / NT : ((n + 31) / 32) * ((n + R - 1) / R);
     return s;
 }
-// Vertex q of those outside the interior vectors; false past the last.
-template <int VW>
-__device__ __forceinline__ bool dif_edge_vertex(const DifSplit &s, int q, int &i, int &j)
+// The single vertex of thread tid in block blk of a field; false past the last.
+template <int VW, bool VEC>
+__host__ __device__ __forceinline__ bool dif_vertex(const DifSplit &s, int blk, int tid, int &i, int &j)
 {
-    const int n = s.n;
-    if (s.nr == 0) {
-        if (q >= n * n) return false;
-        j = q / n;
-        i = q - j * n + 1;
-        j++;
-        return true;
+    if (!VEC) {
+        const int gx = (s.n + 31) / 32, by = blk / gx;
+        i = (blk - by * gx) * 32 + (tid & 31) + 1;
+        j = by * (DIF_NT / 32) + (tid >> 5) + 1;
+        return i <= s.n && j <= s.n;
     }
+    int q = blk * DIF_NT + tid;
+    const int n = s.n;
     const int rows = n - s.nr, top = rows * n;    // the rows below and above the interior rows
     if (q < top) {
         j = q / n;
@@ -233,6 +268,17 @@ __device__ __forceinline__ bool dif_edge_vertex(const DifSplit &s, int q, int &i
     i = q - j * w + 1;
     j += s.lo;
     if (i > s.va * VW) i += s.nv * VW;
+    return true;
+}
+// The first point and the row of the interior vector of thread tid in block blk of a field.
+template <int VW>
+__host__ __device__ __forceinline__ bool dif_vector(const DifSplit &s, int blk, int tid, int &k, int &j)
+{
+    const int q = blk * DIF_NT + tid;
+    if (q >= s.nv * s.nr) return false;
+    const int r = q / s.nv;
+    k = 1 + VW * (s.va + q - r * s.nv);
+    j = s.lo + r;
     return true;
 }
 // x[q] = f(k - R + q), q = 0 .. VW + 2 R - 1, around the vector at p
@@ -254,26 +300,24 @@ __device__ __forceinline__ T dif_d1_in(const T *f)
     else if constexpr (ORD == 42) return (f[0] + T(-8) * f[1] + T(8) * f[3] + -f[4]) / T(12);
     else return (-f[0] + T(9) * f[1] + T(-45) * f[2] + T(45) * f[4] + T(-9) * f[5] + f[6]) / T(60);
 }
-constexpr int DIF_PAIR = 2;   // fields per thread of the interior vectors: the metric is read once for both
-
 // calc_tile_d1x_d1y: d1x = D1x(f) J Qi12, d1y = D1y(f) J Qi12 (sbp_diff_<ORD> node
-// differences).  Grid x: interior blocks, then the others; z: panel + NPAN * (field pair +
-// 2 member).  The point-wise kernel read every stencil input of every vertex by itself
-// (18 loads per vertex and field with the Laplacian's, 13 us per launch at C192 FP32 cold).
-template <class T, int ORD>
-__global__ void __launch_bounds__(256) k_dif_d1(const T *__restrict__ F, T *__restrict__ D1X, T *__restrict__ D1Y, Dims d,
-                                                AhView<T> a, DifSplit sp)
+// differences).  Grid x: the single vertices of two fields, then their interior vectors; z:
+// panel + NPAN * (field pair + 2 member).
+template <class T, int ORD, bool VEC>
+__global__ void __launch_bounds__(DIF_NT) k_dif_d1(const T *__restrict__ F, T *__restrict__ D1X, T *__restrict__ D1Y,
+                                                   Dims d, AhView<T> a, DifSplit sp)
 {
     using V = OV<T>;
     constexpr int VW = V::W, R = (ORD == 21 ? 1 : (ORD == 42 ? 2 : 3));
     const int n = d.N + 1, P = d.P, t = blockIdx.z % NPAN;
-    const int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_PAIR * NPAN * d.ps + t * d.ps;
+    int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_HALF * NPAN * d.ps + t * d.ps;
     pdl_trigger();
-    if ((int)blockIdx.x < sp.ni) {
-        const int q = blockIdx.x * 256 + threadIdx.x;
-        const bool ok = q < sp.nv * sp.nr;
-        const int r = ok ? q / sp.nv : 0, v = sp.va + q - r * sp.nv, j = sp.lo + r;
-        const int64_t o = ok ? box_off(P, 1 + VW * v, j) : 0;
+    if (VEC && (int)blockIdx.x >= DIF_HALF * sp.ne) {
+        int blk = blockIdx.x - DIF_HALF * sp.ne;
+        if (blk >= sp.ni) { blk -= sp.ni; base += NPAN * d.ps; }
+        int k, j;
+        const bool ok = dif_vector<VW>(sp, blk, threadIdx.x, k, j);
+        const int64_t o = ok ? box_off(P, k, j) : 0;
         V J = ov_all(T(0)), Q2 = J;
         if (ok) {
             J = ov_ld(a.J + o);
@@ -281,61 +325,56 @@ __global__ void __launch_bounds__(256) k_dif_d1(const T *__restrict__ F, T *__re
         }
         pdl_wait();
         if (!ok) return;
+        const int64_t b = base + o;
+        const T *f = F + b;
+        T x[VW + 2 * R];
+        dif_row<T, R>(f, x);
+        V y[2 * R + 1], ox, oy;
 #pragma unroll
-        for (int fl = 0; fl < DIF_PAIR; fl++) {
-            const int64_t b = base + (int64_t)fl * NPAN * d.ps + o;
-            const T *f = F + b;
-            T x[VW + 2 * R];
-            dif_row<T, R>(f, x);
-            V y[2 * R + 1], ox, oy;
+        for (int m = 0; m < 2 * R + 1; m++) y[m] = ov_ld(f + (m - R) * P);
 #pragma unroll
-            for (int m = 0; m < 2 * R + 1; m++) y[m] = ov_ld(f + (m - R) * P);
+        for (int e = 0; e < VW; e++) {
+            T c[2 * R + 1];
 #pragma unroll
-            for (int e = 0; e < VW; e++) {
-                T c[2 * R + 1];
-#pragma unroll
-                for (int m = 0; m < 2 * R + 1; m++) c[m] = y[m].a[e];
-                ox.a[e] = dif_d1_in<T, ORD>(x + e) * J.a[e] * Q2.a[e];
-                oy.a[e] = dif_d1_in<T, ORD>(c) * J.a[e] * Q2.a[e];
-            }
-            ov_st(D1X + b, ox);
-            ov_st(D1Y + b, oy);
+            for (int m = 0; m < 2 * R + 1; m++) c[m] = y[m].a[e];
+            ox.a[e] = dif_d1_in<T, ORD>(x + e) * J.a[e] * Q2.a[e];
+            oy.a[e] = dif_d1_in<T, ORD>(c) * J.a[e] * Q2.a[e];
         }
+        ov_st(D1X + b, ox);
+        ov_st(D1Y + b, oy);
         return;
     }
     pdl_wait();
-    int i, j;
-    if (!dif_edge_vertex<VW>(sp, ((int)blockIdx.x - sp.ni) * 256 + threadIdx.x, i, j)) return;
+    int i, j, blk = blockIdx.x;
+    if (blk >= sp.ne) { blk -= sp.ne; base += NPAN * d.ps; }
+    if (!dif_vertex<VW, VEC>(sp, blk, threadIdx.x, i, j)) return;
     const int64_t o = box_off(P, i, j);
     const T J = __ldg(a.J + o), Q2 = __ldg(a.Q2 + o);
-#pragma unroll
-    for (int fl = 0; fl < DIF_PAIR; fl++) {
-        const int64_t b = base + (int64_t)fl * NPAN * d.ps;
-        const GV<T> f{F + b, P};
-        D1X[b + o] = dn2n<T, ORD>(i, n, [&](int k) { return f(k, j); }) * J * Q2;
-        D1Y[b + o] = dn2n<T, ORD>(j, n, [&](int l) { return f(i, l); }) * J * Q2;
-    }
+    const GV<T> f{F + base, P};
+    D1X[base + o] = dn2n<T, ORD>(i, n, [&](int k) { return f(k, j); }) * J * Q2;
+    D1Y[base + o] = dn2n<T, ORD>(j, n, [&](int l) { return f(i, l); }) * J * Q2;
 }
 
 // calc_laplace_tile and divide_by_J_self: the panel-local Laplacian of every vertex; the
 // panel-boundary vertices' values go to R (for the sync), the others to OUT.  The same grid.
-template <class T, int ORD>
-__global__ void __launch_bounds__(256) k_dif_lap(const T *__restrict__ F, const T *__restrict__ D1X,
-                                                 const T *__restrict__ D1Y, T *__restrict__ RAW, T *__restrict__ OUT, Dims d,
-                                                 AhView<T> a, DifView<T> v, DifSplit sp)
+template <class T, int ORD, bool VEC>
+__global__ void __launch_bounds__(DIF_NT, dif_minb<T>(ORD, VEC)) k_dif_lap(
+    const T *__restrict__ F, const T *__restrict__ D1X, const T *__restrict__ D1Y, T *__restrict__ RAW, T *__restrict__ OUT, Dims d,
+    AhView<T> a, DifView<T> v, DifSplit sp)
 {
     using V = OV<T>;
     constexpr int VW = V::W, R = (ORD == 21 ? 1 : (ORD == 42 ? 2 : 3));
     const int n = d.N + 1, P = d.P, t = blockIdx.z % NPAN;
-    const int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_PAIR * NPAN * d.ps + t * d.ps;
+    int64_t base = (int64_t)(blockIdx.z / NPAN) * DIF_HALF * NPAN * d.ps + t * d.ps;
     const T *const w0 = ORD == 21 ? v.w21 : (ORD == 42 ? v.w42 : v.w63);
     const int64_t wd = (int64_t)narrow_width(ORD) * d.ps;   // the y weights follow the x weights
     pdl_trigger();
-    if ((int)blockIdx.x < sp.ni) {
-        const int q = blockIdx.x * 256 + threadIdx.x;
-        const bool ok = q < sp.nv * sp.nr;
-        const int r = ok ? q / sp.nv : 0, vv = sp.va + q - r * sp.nv, j = sp.lo + r;
-        const int64_t o = ok ? box_off(P, 1 + VW * vv, j) : 0;
+    if (VEC && (int)blockIdx.x >= DIF_HALF * sp.ne) {
+        int blk = blockIdx.x - DIF_HALF * sp.ne;
+        if (blk >= sp.ni) { blk -= sp.ni; base += NPAN * d.ps; }
+        int k, j;
+        const bool ok = dif_vector<VW>(sp, blk, threadIdx.x, k, j);
+        const int64_t o = ok ? box_off(P, k, j) : 0;
         V wx[2 * R + 1], wy[2 * R + 1], J = ov_all(T(1));
         if (ok) {
 #pragma unroll
@@ -347,69 +386,63 @@ __global__ void __launch_bounds__(256) k_dif_lap(const T *__restrict__ F, const 
         }
         pdl_wait();
         if (!ok) return;
+        const int64_t b = base + o;
+        const T *f = F + b;
+        T x[VW + 2 * R], z[VW + 2 * R];
+        dif_row<T, R>(f, x);
+        dif_row<T, R>(D1Y + b, z);
+        V y[2 * R + 1], u[2 * R + 1], out;
 #pragma unroll
-        for (int fl = 0; fl < DIF_PAIR; fl++) {
-            const int64_t b = base + (int64_t)fl * NPAN * d.ps + o;
-            const T *f = F + b;
-            T x[VW + 2 * R], z[VW + 2 * R];
-            dif_row<T, R>(f, x);
-            dif_row<T, R>(D1Y + b, z);
-            V y[2 * R + 1], u[2 * R + 1], out;
-#pragma unroll
-            for (int m = 0; m < 2 * R + 1; m++) {
-                y[m] = ov_ld(f + (m - R) * P);
-                u[m] = ov_ld(D1X + b + (m - R) * P);
-            }
-#pragma unroll
-            for (int e = 0; e < VW; e++) {
-                T d2x = wx[0].a[e] * x[e], d2y = wy[0].a[e] * y[0].a[e], c[2 * R + 1];
-#pragma unroll
-                for (int m = 1; m < 2 * R + 1; m++) {
-                    d2x = d2x + wx[m].a[e] * x[e + m];
-                    d2y = d2y + wy[m].a[e] * y[m].a[e];
-                }
-#pragma unroll
-                for (int m = 0; m < 2 * R + 1; m++) c[m] = u[m].a[e];
-                T s = d2x + d2y;
-                s = s + dif_d1_in<T, ORD>(z + e) + dif_d1_in<T, ORD>(c);
-                out.a[e] = s / T(v.h2) / J.a[e];
-            }
-            ov_st(OUT + b, out);
+        for (int m = 0; m < 2 * R + 1; m++) {
+            y[m] = ov_ld(f + (m - R) * P);
+            u[m] = ov_ld(D1X + b + (m - R) * P);
         }
+#pragma unroll
+        for (int e = 0; e < VW; e++) {
+            T d2x = wx[0].a[e] * x[e], d2y = wy[0].a[e] * y[0].a[e], c[2 * R + 1];
+#pragma unroll
+            for (int m = 1; m < 2 * R + 1; m++) {
+                d2x = d2x + wx[m].a[e] * x[e + m];
+                d2y = d2y + wy[m].a[e] * y[m].a[e];
+            }
+#pragma unroll
+            for (int m = 0; m < 2 * R + 1; m++) c[m] = u[m].a[e];
+            T s = d2x + d2y;
+            s = s + dif_d1_in<T, ORD>(z + e) + dif_d1_in<T, ORD>(c);
+            out.a[e] = s / T(v.h2) / J.a[e];
+        }
+        ov_st(OUT + b, out);
         return;
     }
     pdl_wait();
-    int i, j;
-    if (!dif_edge_vertex<VW>(sp, ((int)blockIdx.x - sp.ni) * 256 + threadIdx.x, i, j)) return;
+    int i, j, blk = blockIdx.x;
+    if (blk >= sp.ne) { blk -= sp.ne; base += NPAN * d.ps; }
+    if (!dif_vertex<VW, VEC>(sp, blk, threadIdx.x, i, j)) return;
     // one end's closure block
     constexpr int RC = ORD == 63 ? NarrowBlock<63>::R * NarrowBlock<63>::C : NarrowBlock<42>::R * NarrowBlock<42>::C;
     const T *mb = ORD == 63 ? v.m63 : v.m42;
     const T *wi = w0 + box_off(P, i, j);
     const GV<T> J{a.J, P}, Q1{a.Q1, P}, Q3{a.Q3, P};
-#pragma unroll 1
-    for (int fl = 0; fl < DIF_PAIR; fl++) {
-        const int64_t b = base + (int64_t)fl * NPAN * d.ps;
-        const GV<T> f{F + b, P}, dx1{D1X + b, P}, dy1{D1Y + b, P};
-        T d2x = narrow_d2<T, ORD>(i, n, [&](int k) { return Q1(k, j) * J(k, j); }, [&](int k) { return f(k, j); },
-                                  mb + dif_block_index(n, 0, j, 0, RC), wi, d.ps);
-        const T d2y = narrow_d2<T, ORD>(j, n, [&](int l) { return Q3(i, l) * J(i, l); }, [&](int l) { return f(i, l); },
-                                        mb + dif_block_index(n, 1, i, 0, RC), wi + wd, d.ps);
-        // the boundary penalties 1/h_1 (-+2 d1f), all on d2f_x and in the reference's order
-        const T pen = ORD == 21 ? T(2) : (ORD == 42 ? T(48.0 / 17) : T(43200.0 / 13649));
-        if (i == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dy1(1, j)));
-        if (i == n) d2x = d2x - T(0.5) * (pen * (T(2) * dy1(n, j)));
-        if (j == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dx1(i, 1)));
-        if (j == n) d2x = d2x - T(0.5) * (pen * (T(2) * dx1(i, n)));
-        const T dyx = dn2n<T, ORD>(j, n, [&](int l) { return dx1(i, l); });
-        const T dxy = dn2n<T, ORD>(i, n, [&](int k) { return dy1(k, j); });
-        T r = d2x + d2y;
-        r = r + dxy + dyx;
-        r = r / T(v.h2);
-        r = r / J(i, j);
-        const int64_t o = box_off(P, i, j);
-        if (i == 1 || i == n || j == 1 || j == n) RAW[b + o] = r;
-        else OUT[b + o] = r;
-    }
+    const GV<T> f{F + base, P}, dx1{D1X + base, P}, dy1{D1Y + base, P};
+    T d2x = narrow_d2<T, ORD>(i, n, [&](int k) { return Q1(k, j) * J(k, j); }, [&](int k) { return f(k, j); },
+                              mb + dif_block_index(n, 0, j, 0, RC), wi, d.ps);
+    const T d2y = narrow_d2<T, ORD>(j, n, [&](int l) { return Q3(i, l) * J(i, l); }, [&](int l) { return f(i, l); },
+                                    mb + dif_block_index(n, 1, i, 0, RC), wi + wd, d.ps);
+    // the boundary penalties 1/h_1 (-+2 d1f), all on d2f_x and in the reference's order
+    const T pen = ORD == 21 ? T(2) : (ORD == 42 ? T(48.0 / 17) : T(43200.0 / 13649));
+    if (i == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dy1(1, j)));
+    if (i == n) d2x = d2x - T(0.5) * (pen * (T(2) * dy1(n, j)));
+    if (j == 1) d2x = d2x - T(0.5) * (pen * (T(-2) * dx1(i, 1)));
+    if (j == n) d2x = d2x - T(0.5) * (pen * (T(2) * dx1(i, n)));
+    const T dyx = dn2n<T, ORD>(j, n, [&](int l) { return dx1(i, l); });
+    const T dxy = dn2n<T, ORD>(i, n, [&](int k) { return dy1(k, j); });
+    T r = d2x + d2y;
+    r = r + dxy + dyx;
+    r = r / T(v.h2);
+    r = r / J(i, j);
+    const int64_t o = box_off(P, i, j);
+    if (i == 1 || i == n || j == 1 || j == n) RAW[base + o] = r;
+    else OUT[base + o] = r;
 }
 
 // The Ah scalar sync of the panel-boundary vertices (halo_Ah_scalar_sync_mod.f90:43-98):

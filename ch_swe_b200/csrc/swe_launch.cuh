@@ -77,20 +77,32 @@ static inline cudaError_t set_carveout(K kern)
                           : cudaSuccess;
 }
 
+// Launch after the stream's previous kernel with programmatic serialization; carveout: percent of
+// the SM's L1 kept as shared memory (cudaSharedmemCarveoutDefault: the driver's choice).
 template <typename... KArgs, typename... Args>
-static inline void launch_k(void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t st, Args... args)
+static inline void launch_carveout(int carveout, void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = b;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    if (pdl_enabled()) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (carveout != cudaSharedmemCarveoutDefault) {
+        at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[cfg.numAttrs++].val.sharedMemCarveout = (unsigned)carveout;
+    }
     cudaLaunchKernelEx(&cfg, kern, ((KArgs)args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline void launch_k(void (*kern)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t st, Args... args)
+{
+    launch_carveout(cudaSharedmemCarveoutDefault, kern, g, b, smem, st, args...);
 }
 // Balanced tiles: ceil(N / (TM - 1)) tiles per direction, widths at most TM.
 static inline dim3 stage_grid(int N, int members, int tm)

@@ -68,6 +68,31 @@ def test_apply_parity_fp64_random(order, N):
     dom.destroy()
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("order", [21, 42, 63])
+@pytest.mark.parametrize("N", [31, 32, 33, 34, 35])
+def test_apply_parity_of_vectors_and_single_vertices(order, N, precision):
+    """Every remainder of the vectors' four (FP32) and two (FP64) points; with eight members the
+    interior goes by vectors from C32 on.  FP32: two Laplacians of some 20 terms a
+    point, of the size of the result for random fields, each rounded to 6e-8: 1e-5 in L2."""
+    from ch_swe_b200 import create_stvec_swm, create_swm_diff_operator
+    from oracle.oracle import Oracle
+    st = random_state(N, 300 + N)
+    ref = Oracle(N, h_mean=H).diff_apply(*st, uv_coeff=0.03, h_coeff=0.01, lap_order=order)
+    dom, _ = ah_domain(N, precision, members=8)
+    dif = create_swm_diff_operator(diff_config(order), dom)
+    x, y = create_stvec_swm(dom), create_stvec_swm(dom)
+    for m in range(8):
+        x.upload(*((m + 1) * f for f in st), member=m)
+    dif.apply(y, x, dom)
+    for m in (0, 4, 7):
+        for g, r, name in zip(y.download(member=m), ref, "huv"):
+            r = (m + 1) * r
+            err = rel(g, r) if precision == "fp64" else np.linalg.norm(g - r) / np.linalg.norm(r)
+            assert err < (FP64_RTOL if precision == "fp64" else 1e-5), (order, N, m, name, err)
+    dom.destroy()
+
+
 @pytest.mark.parametrize("order", [21, 42, 63])
 def test_euler_steps_and_driver_loop_fp64(order):
     """Six driver steps on a Gaussian hill: RK4 of the Ah linear operator of the same SBP
