@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(CoLayout<T, XL, TH>::NM)
     }
     __syncwarp();
     if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
-        atomicExch(err, 1);
+        *(volatile int *)err = 1;
         mbar_wait(bar, 0, FUSED_WAIT_NS);
     }
     __syncthreads();
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(TendLayout<T, XL, TH>::NM, 2)
     }
     __syncwarp();
     if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
-        atomicExch(err, 1);
+        *(volatile int *)err = 1;
         mbar_wait(bar, 0, FUSED_WAIT_NS);
     }
     __syncthreads();
@@ -578,7 +578,7 @@ __global__ void __maxnreg__(REGS)
         // the own copy, from the tile's windows (the main threads' arrival: the barrier is initialised)
         nbar_sync(BAR_P2, NM + nband);
         if (!mbar_wait(bar, 0, FUSED_WAIT_NS)) {
-            atomicExch(err, 1);
+            *(volatile int *)err = 1;
             mbar_wait(bar, 0, FUSED_WAIT_NS);
         }
         OneRaw<T> ro{};
@@ -683,7 +683,7 @@ __global__ void __maxnreg__(REGS)
     }
     __syncwarp();
     if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
-        atomicExch(err, 1);
+        *(volatile int *)err = 1;
         mbar_wait(bar, 0, FUSED_WAIT_NS);
     }
     nbar_sync(BAR_MAIN, NM);

@@ -278,7 +278,9 @@ struct swe_ctx {
     int olabel = 0, oocc = 0;
     void *onetab = nullptr;          // OneMetric tables (side lines, edge-vector weights)
     CUtensorMap tm_one;              // TMA map of fmet with the one-launch stage's tiles
-    int *derr = nullptr;             // device error word: a bounded wait in a kernel gave up
+    // error word in pinned host memory, written by a kernel whose bounded wait for its tile
+    // loads gave up; set until swe_synchronize has reported it
+    int *derr = nullptr;
     bool launch_miss = false;        // a stage or contravariant launch found no built configuration
     bool graph_members = false;      // the cached graph uses the per-member time steps
     double *dtm = nullptr;           // per-member time steps (device), swe_rk4_steps_members
@@ -361,6 +363,16 @@ static cudaError_t clear_device(swe_ctx *c, void *p, size_t bytes)
 {
     cudaError_t e = cudaMemsetAsync(p, 0, bytes, c->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
+// Wait for the context's work, for a call that returns its results: an error where a kernel gave
+// up waiting for its tile loads.  Every such call reports it until swe_synchronize has.
+static int results_ready(swe_ctx *c)
+{
+    CU(c, cudaStreamSynchronize(c->stream));
+    if (*(volatile int *)c->derr)
+        return fail(c, SWE_ECUDA, "a stage kernel gave up waiting for its tile loads; its outputs are incomplete");
+    return SWE_OK;
 }
 
 static bool g_tables_ready[64] = {false};
@@ -1090,8 +1102,9 @@ static void free_ctx(swe_ctx *c)
     cudaFree(c->fl); cudaFree(c->adt); cudaFree(c->fs); cudaFree(c->vh); cudaFree(c->ones); cudaFree(c->hb);
     cudaFree(c->ah64.base); cudaFree(c->ah32.base); cudaFree(c->qa); cudaFree(c->negones);
     cudaFree(c->dif); cudaFree(c->dif_b);
-    cudaFree(c->fmet); cudaFree(c->onetab); cudaFree(c->derr); cudaFree(c->hs); cudaFree(c->cmet);
+    cudaFree(c->fmet); cudaFree(c->onetab); cudaFree(c->hs); cudaFree(c->cmet);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->derr) cudaFreeHost(c->derr);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     if (c->side) cudaStreamDestroy(c->side);
     for (cudaEvent_t e : {c->ev_fork, c->ev_havg, c->ev_co2, c->ev_side})
@@ -1197,8 +1210,8 @@ extern "C" int swe_ctx_create(const swe_cfg *cfg, swe_ctx **out)
     c->Hhost.assign(cfg->n_members, cfg->h_mean);
     if (cudaMalloc(&c->Hm, sizeof(double) * cfg->n_members) != cudaSuccess) return bail(SWE_ENOMEM);
     if (cudaMalloc(&c->dtm, sizeof(double) * cfg->n_members) != cudaSuccess) return bail(SWE_ENOMEM);
-    if (cudaMalloc(&c->derr, sizeof(int)) != cudaSuccess) return bail(SWE_ENOMEM);
-    if (clear_device(c, c->derr, sizeof(int)) != cudaSuccess) return bail(SWE_ECUDA);
+    if (cudaHostAlloc((void **)&c->derr, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return bail(SWE_ENOMEM);
+    *c->derr = 0;
     if (to_device(c, c->Hm, c->Hhost.data(), sizeof(double) * cfg->n_members) != cudaSuccess)
         return bail(SWE_ECUDA);
     if ((rc = alloc_box(c, &c->ya)) || (rc = alloc_box(c, &c->yb)) || (rc = alloc_box(c, &c->acc)) ||
@@ -1272,15 +1285,9 @@ extern "C" int swe_set_stream(swe_ctx *c, void *s)
 extern "C" int swe_synchronize(swe_ctx *c)
 {
     if (!c) return SWE_EINVAL;
-    CU(c, cudaStreamSynchronize(c->stream));
-    // a kernel whose bounded wait for its tile loads ran out leaves a flag behind
-    int flag = 0;
-    CU(c, cudaMemcpy(&flag, c->derr, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) {
-        CU(c, clear_device(c, c->derr, sizeof(int)));
-        return fail(c, SWE_ECUDA, "a stage kernel gave up waiting for its tile loads; its outputs are incomplete");
-    }
-    return SWE_OK;
+    const int rc = results_ready(c);
+    *c->derr = 0;
+    return rc;
 }
 
 extern "C" long long swe_launch_count(const swe_ctx *c) { return c ? c->launches : -1; }
@@ -1467,7 +1474,7 @@ static int download_range(const swe_stvec *vec, int m0, int count, double *h, do
     const size_t mbytes = (size_t)c->dims.ms * c->elem;
     unsigned char *buf = c->pinned;
     CU(c, cudaMemcpyAsync(buf, (char *)vec->d + m0 * mbytes, mbytes * count, cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     panel_tasks(count, c->cfg.N, [&](int k, int t) {
         if (c->elem == 8)
             unpack_panel<double>(c, (const double *)(buf + k * mbytes), h + k * nh, u + k * nu, v + k * nu, t);
@@ -2550,7 +2557,7 @@ extern "C" int swe_integrals(swe_ctx *c, const swe_stvec *vec, int member, doubl
         CU_LAUNCHED(c);
         std::vector<double> part(nb * 3);
         CU(c, cudaMemcpyAsync(part.data(), c->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        CU(c, cudaStreamSynchronize(c->stream));
+        if (int ready = results_ready(c)) return ready;
         double sum[3] = {0, 0, 0};
         for (int q = 0; q < 3; q++)
             for (int k = 0; k < nb; k++) sum[q] += part[q * nb + k];
@@ -2576,7 +2583,7 @@ extern "C" int swe_integrals(swe_ctx *c, const swe_stvec *vec, int member, doubl
     CU_LAUNCHED(c);
     std::vector<double> part(nb * 4);
     CU(c, cudaMemcpyAsync(part.data(), c->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     double s[4] = {0, 0, 0, 0};
     for (int q = 0; q < 4; q++)
         for (int k = 0; k < nb; k++) s[q] += part[q * nb + k];
@@ -2647,7 +2654,7 @@ extern "C" int swe_diag(swe_ctx *c, const swe_stvec *vec, int member, double dt,
     CU_LAUNCHED(c);
     std::vector<double> part(nb * 4);
     CU(c, cudaMemcpyAsync(part.data(), c->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     double hmax = -INFINITY, hmin = INFINITY, umax = 0.0, vmax = 0.0;
     for (int k = 0; k < nb; k++) {
         hmax = std::max(hmax, part[k]);
@@ -2842,7 +2849,7 @@ extern "C" int swe_curl(swe_ctx *c, const swe_stvec *vec, int member, double *ou
     c->launches += 1;
     CU_LAUNCHED(c);
     CU(c, cudaMemcpyAsync(out, dcurl, ncurl * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     return SWE_OK;
 }
 
@@ -2870,7 +2877,7 @@ extern "C" int swe_energies(swe_ctx *c, const swe_stvec *vec, int member, double
     CU_LAUNCHED(c);
     std::vector<double> part(nb * 4);
     CU(c, cudaMemcpyAsync(part.data(), c->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     double sum[4] = {0, 0, 0, 0};
     for (int q = 0; q < 4; q++)
         for (int k = 0; k < nb; k++) sum[q] += part[q * nb + k];
@@ -3485,7 +3492,7 @@ extern "C" int swe_regrid_latlon(swe_ctx *c, const swe_stvec *vec, int member, i
         c->launches += 3;
         CU_LAUNCHED(c);
         CU(c, cudaMemcpyAsync(out, dout, (size_t)np * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        CU(c, cudaStreamSynchronize(c->stream));
+        if (int ready = results_ready(c)) return ready;
         return SWE_OK;
     }
     int rc = ensure_latlon(c, nlat, nlon);
@@ -3511,7 +3518,7 @@ extern "C" int swe_regrid_latlon(swe_ctx *c, const swe_stvec *vec, int member, i
     c->launches += 2;
     CU_LAUNCHED(c);
     CU(c, cudaMemcpyAsync(out, dout, (size_t)np * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     return SWE_OK;
 }
 
@@ -3544,7 +3551,7 @@ extern "C" int swe_regrid_latlon_wind(swe_ctx *c, const swe_stvec *vec, int memb
     CU_LAUNCHED(c);
     CU(c, cudaMemcpyAsync(u_out, uo, (size_t)np * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CU(c, cudaMemcpyAsync(v_out, vo, (size_t)np * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(c, cudaStreamSynchronize(c->stream));
+    if (int ready = results_ready(c)) return ready;
     return SWE_OK;
 }
 
@@ -3634,7 +3641,7 @@ extern "C" int swe_kernel_times(swe_ctx *c, swe_stvec *v0, double dt, int nreps,
                 timed_stage<float>(c, c->m32.v, bufs_in[s], v0->d, bufs_out[s], v0->cmp, s + 1, dt, e[0], e[1], e[2], e[3]);
         }
     CU_LAUNCHED(c);
-    CU(c, cudaStreamSynchronize(c->stream));
+    if ((rc = results_ready(c))) return rc;
     double t_co = 0.0, t_ed = 0.0, t_st = 0.0;
     for (int q = 0; q < nst; q++) {
         float a = 0.f, b = 0.f, d = 0.f;
@@ -3999,7 +4006,8 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
             return SWE_OK;
         }
     swe_stvec *v = nullptr;
-    int rc = swe_stvec_create(c, &v);
+    int rc = results_ready(c);   // an error word set below is a candidate's
+    if (rc == SWE_OK) rc = swe_stvec_create(c, &v);
     if (rc) return rc;
     const int keep_tile = c->one ? c->olabel : (c->fused ? c->fth : c->tile),
               keep_occ = c->one ? c->oocc : (c->fused ? c->focc : c->occ), keep_runs = c->one ? 3 : (c->fused ? 2 : c->runs);
@@ -4056,6 +4064,10 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
             cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
             rc = fail(c, SWE_ECUDA, "autotune timing");
             break;
+        }
+        if (*(volatile int *)c->derr) {   // a candidate whose tile loads do not arrive
+            *c->derr = 0;
+            continue;
         }
         const double m = t / nreps;
         const int ti = kc.tile == 17 ? 0 : (kc.tile == 25 ? 1 : 2);

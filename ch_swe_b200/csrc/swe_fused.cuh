@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, OCC)
         // the tile loads did not arrive: record it and leave (after one more bounded
         // wait, so that no copy is still writing this block's shared memory)
         if (threadIdx.x == 0) {
-            atomicExch(err, 1);
+            *(volatile int *)err = 1;
             mbar_wait(bar, 0, FUSED_WAIT_NS);
         }
         return;

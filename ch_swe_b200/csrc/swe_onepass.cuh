@@ -545,7 +545,7 @@ __global__ void __maxnreg__(REGS)
     if (tid < 32 && !mbar_wait(bar, 0, FUSED_WAIT_NS)) {
         // the tile loads did not arrive: record it, wait once more (bounded), and finish on
         // whatever the windows hold
-        atomicExch(err, 1);
+        *(volatile int *)err = 1;
         mbar_wait(bar, 0, FUSED_WAIT_NS);
     }
     nbar_sync(BAR_MAIN, NM);
