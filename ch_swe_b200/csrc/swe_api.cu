@@ -274,6 +274,7 @@ struct swe_ctx {
     // one-launch stage (swe_onepass.cuh) of the linear Ch 4-2 operator: selected instead of
     // the split kernels and the fused stage when `one`; (olabel, oocc) is its configuration.
     // A context of that operator starts with it (`one_default`) until a configuration is set.
+    // The split configuration above stays beside it: what the context runs in a group.
     bool one = false, one_default = false;
     int olabel = 0, oocc = 0;
     void *onetab = nullptr;          // OneMetric tables (side lines, edge-vector weights)
@@ -2087,8 +2088,8 @@ extern "C" int swe_group_create(swe_ctx *const *ctxs, int n, swe_group **out)
             return fail(c0, SWE_EINVAL, "group: context %d has another device or precision than context 0", k);
         if (c->adv || c->ah || c->cstag || c->ord != 42)
             return fail(c0, SWE_EINVAL, "group: context %d is not the linear operator on Ch in SBP 4-2", k);
-        // a context on its default stage joins with its split configuration
-        if (c->fused || (c->one && !c->one_default) || c->tile != c0->tile || c->occ != c0->occ || c->runs != c0->runs)
+        // a context on the vector stage joins with its split configuration
+        if (c->fused || c->tile != c0->tile || c->occ != c0->occ || c->runs != c0->runs)
             return fail(c0, SWE_EINVAL, "group: context %d has another kernel configuration than context 0 "
                         "(the contexts share one split configuration)", k);
     }
@@ -2211,7 +2212,7 @@ extern "C" int swe_group_rk4_steps_members(swe_group *g, swe_stvec *const *state
             if (!(dt[k][m] >= 0.0) || !std::isfinite(dt[k][m]))
                 return gfail(g, SWE_EINVAL, "group: context %d member %d: time step %g (need finite, >= 0)", k, m,
                              dt[k][m]);
-        if (c->fused || (c->one && !c->one_default) || c->tile != g->tile || c->occ != g->occ || c->runs != g->runs)
+        if (c->fused || c->tile != g->tile || c->occ != g->occ || c->runs != g->runs)
             return gfail(g, SWE_EINVAL, "group: context %d changed its kernel configuration", k);
     }
     if (nsteps == 0) return SWE_OK;
@@ -3974,12 +3975,20 @@ struct TuneKey {
 };
 struct TuneEntry {
     TuneKey key;
-    int tile, occ, runs;
+    KernelCfg best, split;   // the fastest configuration, and the fastest of the split kernels
     double ms[3];
     bool branches;
 };
 std::vector<TuneEntry> g_tuned;   // process-wide results of swe_autotune
 }  // namespace
+
+// Configuration k, with `split` as the configuration of the split kernels beside it (groups, the
+// diagnostics' contravariant components) where k is another stage's.
+static int apply_tuned(swe_ctx *c, const KernelCfg &k, const KernelCfg &split)
+{
+    if (k.runs >= 2) set_cfg(c, split.tile, split.occ, split.runs);
+    return apply_cfg(c, k.tile, k.occ, k.runs);
+}
 
 // Time RK4 steps of a zero state for every built kernel configuration (tile edge
 // and blocks per SM; the advective operator's stage kernel exists for one
@@ -3998,10 +4007,10 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
     const TuneKey key{c->device, c->cfg.N, c->cfg.precision, c->cfg.n_members, c->cfg.operator_kind, c->ord};
     for (const TuneEntry &e : g_tuned)
         if (e.key == key) {
-            if (int rc = apply_cfg(c, e.tile, e.occ, e.runs)) return rc;
+            if (int rc = apply_tuned(c, e.best, e.split)) return rc;
             if (c->branches != e.branches) drop_graph(c);
             c->branches = e.branches;
-            if (best_tile) *best_tile = e.tile;
+            if (best_tile) *best_tile = e.best.tile;
             if (ms_per_step) for (int k = 0; k < 3; k++) ms_per_step[k] = e.ms[k];
             return SWE_OK;
         }
@@ -4009,12 +4018,12 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
     int rc = results_ready(c);   // an error word set below is a candidate's
     if (rc == SWE_OK) rc = swe_stvec_create(c, &v);
     if (rc) return rc;
-    const int keep_tile = c->one ? c->olabel : (c->fused ? c->fth : c->tile),
-              keep_occ = c->one ? c->oocc : (c->fused ? c->focc : c->occ), keep_runs = c->one ? 3 : (c->fused ? 2 : c->runs);
+    const KernelCfg keep_split{c->tile, c->occ, c->runs},
+        keep = c->one ? KernelCfg{c->olabel, c->oocc, 3} : (c->fused ? KernelCfg{c->fth, c->focc, 2} : keep_split);
     const bool keep_default = c->one_default;
     double ms[3] = {1e300, 1e300, 1e300};
-    int best_t = keep_tile, best_o = keep_occ, best_r = keep_runs;
-    double best_ms = 1e300;
+    KernelCfg best = keep, split = keep_split;
+    double best_ms = 1e300, split_ms = 1e300;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     rc = SWE_OK;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) rc = fail(c, SWE_ECUDA, "autotune events");
@@ -4072,13 +4081,14 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
         const double m = t / nreps;
         const int ti = kc.tile == 17 ? 0 : (kc.tile == 25 ? 1 : 2);
         ms[ti] = std::min(ms[ti], m);
-        if (m < best_ms) { best_ms = m; best_t = kc.tile; best_o = kc.occ; best_r = kc.runs; }
+        if (m < best_ms) { best_ms = m; best = kc; }
+        if (kc.runs < 2 && m < split_ms) { split_ms = m; split = kc; }
     }
     // advective operator: the best configuration with the stage forked onto the side
     // stream and on one stream (forking pays for small cubes, not always for C384)
     bool best_b = c->branches;
     if (rc == SWE_OK && c->side) {
-        apply_cfg(c, best_t, best_o, best_r);
+        apply_tuned(c, best, split);
         double tb[2] = {1e300, 1e300};
         for (int b = 0; b < 2 && rc == SWE_OK; b++) {
             drop_graph(c);
@@ -4101,14 +4111,14 @@ extern "C" int swe_autotune(swe_ctx *c, int nreps, int *best_tile, double *ms_pe
     swe_stvec_destroy(v);
     drop_graph(c);
     if (rc != SWE_OK) {
-        apply_cfg(c, keep_tile, keep_occ, keep_runs);
+        apply_tuned(c, keep, keep_split);
         c->one_default = keep_default;
         return rc;
     }
-    if ((rc = apply_cfg(c, best_t, best_o, best_r)) != SWE_OK) return rc;
-    TuneEntry te{key, best_t, best_o, best_r, {ms[0], ms[1], ms[2]}, best_b};
+    if ((rc = apply_tuned(c, best, split)) != SWE_OK) return rc;
+    TuneEntry te{key, best, split, {ms[0], ms[1], ms[2]}, best_b};
     g_tuned.push_back(te);
-    if (best_tile) *best_tile = best_t;
+    if (best_tile) *best_tile = best.tile;
     if (ms_per_step) for (int k = 0; k < 3; k++) ms_per_step[k] = ms[k];
     return SWE_OK;
 }

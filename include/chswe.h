@@ -172,8 +172,12 @@ int swe_rk4_steps_members(swe_ctx *ctx, swe_stvec *v0, const double *dt, int nst
    kernel configuration (17, 4, 0), (25, 3, 0) or (33, 2, 0) -- launched as one grid
    per kernel: twelve launches per RK4 step whatever the number of contexts, on the
    first context's stream, ordered after the work queued on every context's stream
-   and before the work queued there later.  A context advanced in a group gets the
-   bits it gets from swe_rk4_steps_members with the same configuration.  The group
+   and before the work queued there later.  A context whose stage is the vector stage
+   (runs 3) joins with the split configuration it keeps beside it: the one set last,
+   else the context's first (swe_set_tile), else the autotuner's fastest; a context on
+   the fused stage (runs 2) is refused.  A context advanced in a group gets the bits
+   it gets from swe_rk4_steps_members with the split configuration set, which differ in
+   rounding from the vector stage's.  The group
    uses each context's scratch and per-member time-step buffer: a context takes no
    other calls while its group's steps may be in flight on another stream, and
    outlives its group.  No reference counterpart: the reference advances one state per

@@ -96,3 +96,61 @@ def test_group_refuses_mismatched_domains():
         create_group([a])
     for x in (a, b, c, d):
         x.destroy()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_a_context_on_the_vector_stage_joins_with_its_split_configuration(precision):
+    """The vector stage, by default or by name, keeps the split configuration beside it; in the
+    group the context gets the bits of that configuration."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    from ch_swe_b200.swm import create_group
+    N, dts = 40, np.array([120.0])
+    rng = np.random.default_rng(3)
+    from ch_swe_b200 import state_shapes
+    ic = [rng.standard_normal(s) for s in state_shapes(N)]
+    out = []
+    for stage in ((25, 3, 0), (33, 2 if precision == "fp32" else 1, 3)):
+        dom = create_domain(N, precision=precision)
+        dom.kernel_config = (25, 3, 0)
+        dom.kernel_config = stage
+        op = create_swm_operator(dom.grav, {"swm_operator_type": "linear_swm_operator", "h_mean": 1000.0}, dom)
+        st = create_stvec_swm(dom).upload(*ic)
+        if stage[2] == 3:
+            grp = create_group([dom])
+            grp.steps_members([st], [dts], 9)
+            grp.synchronize()
+            assert dom.kernel_config == stage
+            grp.destroy()
+        else:
+            create_timescheme(st, "rk4").steps_members(st, op, dts, 9)
+        out.append(st.download())
+        dom.destroy()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_autotuned_contexts_keep_one_split_configuration(precision):
+    """A context that measured and one that takes the measurement from the cache are alike: they
+    share a group (where their split configuration has a group launch), and their diagnostics,
+    which run the split kernels, have the same bits."""
+    from ch_swe_b200 import SweError, create_domain, create_stvec_swm, create_swm_operator, state_shapes
+    from ch_swe_b200.swm import create_group
+    N = 43
+    rng = np.random.default_rng(4)
+    ic = [rng.standard_normal(s) for s in state_shapes(N)]
+    doms, sums = [], []
+    for _ in range(2):
+        dom = create_domain(N, precision=precision)
+        dom.autotune(nreps=4)
+        op = create_swm_operator(dom.grav, {"swm_operator_type": "linear_swm_operator", "h_mean": 1000.0}, dom)
+        sums.append(op.integrals(create_stvec_swm(dom).upload(*ic)))
+        doms.append(dom)
+    assert doms[0].kernel_config == doms[1].kernel_config and sums[0] == sums[1]
+    if doms[0].kernel_config[2] != 2:
+        try:
+            create_group(doms).destroy()
+        except SweError as e:
+            assert "has no group launch" in str(e), e
+    for d in doms:
+        d.destroy()
