@@ -1123,9 +1123,10 @@ static int alloc_box(swe_ctx *c, void **p)
 template <class T>
 static cudaError_t stage_smem_optin();
 
-// The vector stage's configuration a Ch 4-2 context starts with; tile 0: the split kernels.
-// Cubes below 16 cells keep the split kernels and their twelve launches a step, which
-// swe_launch_count reports there.
+// The vector stage's configuration a Ch 4-2 context starts with; tile 0: the split kernels, where
+// no tile of the configuration fits the register file (blocks that touch four sides: linear FP64
+// below C13, and some larger member counts up to C16).  Small cubes, linear, alone, split /
+// vector, us per RK4 step: C8 FP32 61 / 19, C15 FP32 65 / 19, C15 FP64 71 / 20.
 //   FP32: tiles of 7 vectors by 28 rows at every size (measured per RK4 step, alone: C48 / C96 /
 //   C192 / C384 19.9 / 22.6 / 30.6 / 97.5 us against 75 / 80 / 86 / 176 us of the best split or
 //   fused configuration; 256 x C48 576 against 1139 us).
@@ -1138,7 +1139,6 @@ static KernelCfg one_default_cfg(int N, int members, bool adv)
 {
     OneGrid og;
     const KernelCfg none{0, 0, 0};
-    if (N < 16) return none;
     if (adv) {
         // FP64, alone, per RK4 step with (17, 2) / (25, 2) / (33, 1): C96 104 / 99 / 101 us, C192
         // 171 / 197 / 159, C384 407 / 432 / 431
@@ -1685,7 +1685,7 @@ static void launch_adv(swe_ctx *c, const void *yin, const AdvView<T> &av, const 
                  (const T *)c->w, (const T *)c->vh, (T *)c->adt, c->dims, av, mv, dtm);
 }
 
-// One stage of the advective operator through its vector kernels (swe_advone.cuh), six
+// One stage of the advective operator through its vector kernels (swe_advone.cuh), five
 // launches; false: a tensor map cannot be encoded and nothing was launched.
 template <class T>
 static bool enqueue_adv_one(swe_ctx *c, const void *yin, void *v0, void *y1, void *acc, float *cmp, int mode, double dt,

@@ -191,7 +191,7 @@ class Domain:
         thread evaluates runs of consecutive outputs along a stencil; runs 2: the fused
         stage (contravariant components computed in the stage kernel, TMA-loaded tiles of
         at most 26 columns and `tile` rows); runs 3: the vector stage (one launch per RK
-        stage of the linear operator, six of the advective one; the default)."""
+        stage of the linear operator, five of the advective one; the default)."""
         t, o, r = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(_lib.load().swe_get_kernel_config(self.ctx, ctypes.byref(t), ctypes.byref(o), ctypes.byref(r)),
               self.ctx, "swe_get_kernel_config")

@@ -290,8 +290,9 @@ int swe_get_tile(const swe_ctx *ctx, int *tile);
    (33, 3), each with runs 0 and 1; swe_set_tile picks (17, 3, 0), (25, 2, 0) or
    (33, 2, 0).  The advective operator's stage kernel always uses the tile's first
    blocks-per-SM value.  runs 2: the fused stage (linear operator, Ch, SBP 4-2).  runs 3:
-   the vector stage of Ch contexts in SBP 4-2, the default from 16 cells on -- linear
-   operator one launch per RK stage, advective six; tile is at least the rows of its
+   the vector stage of Ch contexts in SBP 4-2, the default where one of its tiles suits
+   the cube (linear FP64: from 13 cells on, with some exceptions below 26) -- linear
+   operator one launch per RK stage, advective five; tile is at least the rows of its
    tiles.  Linear FP32 (17, 2), (25, 2), (33, 2), FP64 (17, 1), (25, 1), (33, 1);
    advective FP32 (25, 2), (33, 2), FP64 (17, 2), (25, 2), (33, 1); a configuration that
    the cube's tiles do not suit returns SWE_EINVAL.  No reference counterpart. */

@@ -177,3 +177,30 @@ def test_advective_members_share_the_halo_launch(N, cfg):
     for f in range(3):
         assert np.array_equal(out[f][1], stack[f][1])
     dom.destroy()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("operator", ["linear", "advective"])
+@pytest.mark.parametrize("N", [8, 9, 10, 11, 12, 13, 14, 15])
+def test_default_stage_of_the_smallest_cubes(N, operator, precision):
+    """Below 16 cells too a context starts on the vector stage where a configuration's blocks fit
+    (linear FP64: from 13 cells on); members with their own time steps against the oracle."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    from oracle.oracle import Oracle
+    M = 2
+    states = [random_state(N, 10 * N + k) for k in range(M)]
+    stack = [np.stack([s[f] + (1000.0 if operator == "advective" and f == 0 else 0.0) for s in states]) for f in range(3)]
+    dts = np.array([60.0, 30.0])
+    dom = create_domain(N, precision=precision, n_members=M, operator=operator, h_mean=1000.0)
+    assert (dom.kernel_config[2] == 3) == (operator == "advective" or precision == "fp32" or N >= 13)
+    op = create_swm_operator(dom.grav, {"swm_operator_type": operator + "_swm_operator", "h_mean": 1000.0}, dom)
+    st = create_stvec_swm(dom).upload(*stack, member=None)
+    create_timescheme(st, "rk4").steps_members(st, op, dts, 3)
+    dom.synchronize()
+    out = st.download(member=None)
+    o = Oracle(N, h_mean=1000.0, operator=operator)
+    for m in range(M):
+        ref = o.rk4(*(f[m] for f in stack), dts[m], 3)
+        for g, r, name in zip(out, ref, "huv"):
+            assert rel(g[m], r) < RTOL[precision], (m, name, rel(g[m], r))
+    dom.destroy()
