@@ -1127,30 +1127,46 @@ static cudaError_t stage_smem_optin();
 // no tile of the configuration fits the register file (blocks that touch four sides: linear FP64
 // below C13, and some larger member counts up to C16).  Small cubes, linear, alone, split /
 // vector, us per RK4 step: C8 FP32 61 / 19, C15 FP32 65 / 19, C15 FP64 71 / 20.
-//   FP32: tiles of 7 vectors by 28 rows at every size (measured per RK4 step, alone: C48 / C96 /
-//   C192 / C384 19.9 / 22.6 / 30.6 / 97.5 us against 75 / 80 / 86 / 176 us of the best split or
-//   fused configuration; 256 x C48 576 against 1139 us).
-//   FP64: full-width tiles for many members of a cube that one tile spans (64 x C48: 318 us
-//   against 371 with the large tiles and 425 split: fewer panel corners per block); tiles of 10
-//   vectors by 25 rows where they make at most one wave (C96: 27.4 against 29.0 us); else 14
-//   vectors by 28 rows (C192 69 against 102 us split, C384 213 against 265 us fused).
+// us per RK4 step, alone:
+//   Linear FP32: tiles of 7 vectors by 28 rows at every size (C48 / C96 / C192 / C384 19.9 / 22.6 /
+//   30.6 / 97.5 against 75 / 80 / 86 / 176 of the best split or fused configuration; 256 x C48
+//   576 against 1139).
+//   Linear FP64: full-width tiles for several members of a cube that one tile spans (64 x C48
+//   305 against 389 with (25, 1), 351 with (33, 1) and 448 split: fewer panel corners per block).
+//   Below C26 only while the panels make one wave: beyond it (25, 1), where it fits (64 x C24 157
+//   / 195 / 184 with (25, 1) / (17, 1) / split), else split from two waves on (128 x C18 330 /
+//   260 with (17, 1) / split, 16 x C18 58 / 85).  A few members of larger cubes: tiles of 10
+//   vectors by 25 rows where they make at most one wave (C96: 27.4 against 29.0), else 14 vectors by
+//   28 rows (C192 69 against 102 split, C384 213 against 265 fused).
+//   Advective FP64: (25, 2) for several members of small cubes, otherwise the largest tiles,
+//   (33, 1), where they make at most one wave, else (17, 2); with (17, 2) / (25, 2) / (33, 1): 16 x
+//   C36 208 / 190 / 217, 4 x C64 170 / 158 / 169, 4 x C96 209 / 211 / 260, one cube C48 77 / 77 / 75, C96 94 / 94 / 86, C108 89 / 94 / 81, C112 106 /
+//   108 / 152, C128 138 / 164 / 177, C144 174 / 173 / 165, C160 179 / 152 / 187, C192 164 / 166 / 189, C256 223 / 221 / 255,
+//   C384 405 / 455 / 459, 16 x C80 443 / 486 / 453.
+//   Advective FP32: (33, 2), but (25, 2), 13 vectors by 18 rows, for one cube that two such tiles
+//   span; with (25, 2) / (33, 2): C52 74 / 73, C56 66 / 78, C64 70 / 87, C80 93 / 108, C96 82 / 85,
+//   C104 81 / 79, C192 103 / 97, 4 x C64 112 / 109, 16 x C80 333 / 293.
+constexpr int ONE_WAVE = 148;   // blocks of a kernel that takes an SM each
 template <class T>
 static KernelCfg one_default_cfg(int N, int members, bool adv)
 {
     OneGrid og;
+    auto blocks = [&] { return (long long)og.g.x * og.g.y * og.g.z; };
     const KernelCfg none{0, 0, 0};
     if (adv) {
-        // FP64, alone, per RK4 step with (17, 2) / (25, 2) / (33, 1): C96 104 / 99 / 101 us, C192
-        // 171 / 197 / 159, C384 407 / 432 / 431
-        const KernelCfg k = sizeof(T) == 4 ? KernelCfg{33, 2, 3}
-                                           : (N < 128 ? KernelCfg{25, 2, 3} : (N < 256 ? KernelCfg{33, 1, 3} : KernelCfg{17, 2, 3}));
+        const bool wave = sizeof(T) == 8 && AdvOneTU<T>::grid(33, 1, N, members, og) && blocks() <= ONE_WAVE;
+        const KernelCfg k = sizeof(T) == 4 ? (members == 1 && N > 52 && N <= 100 ? KernelCfg{25, 2, 3} : KernelCfg{33, 2, 3})
+                            : members > 1 && N <= 64 ? KernelCfg{25, 2, 3} : (wave ? KernelCfg{33, 1, 3} : KernelCfg{17, 2, 3});
         return AdvOneTU<T>::grid(k.tile, k.occ, N, members, og) ? k : none;
     }
     if (sizeof(T) == 4) return OneTU<T>::grid(33, 2, N, members, og) ? KernelCfg{33, 2, 3} : none;
-    if (members > 4 && OneTU<T>::grid(17, 1, N, members, og) && og.g.x == 1) return KernelCfg{17, 1, 3};
+    if (members > 4 && OneTU<T>::grid(17, 1, N, members, og) && og.g.x == 1) {
+        if (N >= 26 || NPAN * members <= ONE_WAVE) return KernelCfg{17, 1, 3};
+        if (OneTU<T>::grid(25, 1, N, members, og)) return KernelCfg{25, 1, 3};
+        return NPAN * members <= 2 * ONE_WAVE ? KernelCfg{17, 1, 3} : none;
+    }
     for (int label : {25, 33})
-        if (OneTU<T>::grid(label, 1, N, members, og) && (og.g.x * og.g.y * og.g.z <= 148 || label == 33))
-            return KernelCfg{label, 1, 3};
+        if (OneTU<T>::grid(label, 1, N, members, og) && (blocks() <= ONE_WAVE || label == 33)) return KernelCfg{label, 1, 3};
     return none;
 }
 

@@ -204,3 +204,18 @@ def test_default_stage_of_the_smallest_cubes(N, operator, precision):
         for g, r, name in zip(out, ref, "huv"):
             assert rel(g[m], r) < RTOL[precision], (m, name, rel(g[m], r))
     dom.destroy()
+
+
+@pytest.mark.parametrize("operator,precision,N,members,cfg", [
+    ("linear", "fp64", 18, 16, (17, 1, 3)), ("linear", "fp64", 18, 64, (25, 2, 0)), ("linear", "fp64", 24, 64, (25, 1, 3)),
+    ("linear", "fp64", 26, 64, (17, 1, 3)), ("linear", "fp64", 96, 1, (25, 1, 3)), ("linear", "fp64", 192, 1, (33, 1, 3)),
+    ("linear", "fp32", 192, 1, (33, 2, 3)), ("advective", "fp64", 108, 1, (33, 1, 3)), ("advective", "fp64", 128, 1, (17, 2, 3)),
+    ("advective", "fp64", 64, 4, (25, 2, 3)), ("advective", "fp64", 80, 16, (17, 2, 3)), ("advective", "fp32", 52, 1, (33, 2, 3)), ("advective", "fp32", 80, 1, (25, 2, 3)),
+    ("advective", "fp32", 80, 4, (33, 2, 3)), ("advective", "fp32", 128, 1, (33, 2, 3))])
+def test_default_configuration(operator, precision, N, members, cfg):
+    """The configuration a context starts with, on both sides of each line of the rule: the
+    sizes at which another one was measured slower than the split kernels are among them."""
+    from ch_swe_b200 import create_domain
+    dom = create_domain(N, precision=precision, n_members=members, operator=operator)
+    assert dom.kernel_config == cfg
+    dom.destroy()
