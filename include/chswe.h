@@ -133,7 +133,10 @@ int swe_stvec_update(swe_stvec *y, double s1, const swe_stvec *v1, double s2, co
    point (i, j) (1-based) at row j+3, column i+3; the 4-point margins hold zeros. */
 int swe_stvec_device_view(const swe_stvec *vec, void **ptr, size_t *bytes, int *precision, int *pitch);
 
-/* vout = A(vin), A the linear shallow-water operator. */
+/* vout = A(vin), A the linear shallow-water operator.  An infinity or NaN of vin reaches every
+   output whose stencil reads it; on the fused and vector stages (runs 2 and 3) also outputs
+   beside a panel edge within eight points of it, whose closure rows carry it with a weight of
+   zero.  The same holds for the steps. */
 int swe_operator_apply(swe_ctx *ctx, swe_stvec *vout, const swe_stvec *vin);
 /* vout.u, vout.v = contravariant components (ut, vt) of vin's covariant wind; vout.h unchanged.
    Mirrors co2contra_operator_t%transform (co2contra_Ch_mod.f90:27-94). */
