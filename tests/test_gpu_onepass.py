@@ -6,6 +6,8 @@ FP64), with one, two and several tiles per direction.  Random states: the duplic
 vertices and both winds disagree across the panels.  Tolerances as for the other stage
 kernels: FP64 within 1e-12 relative (max-norm) of the oracle, FP32 within 1e-5.
 """
+import functools
+
 import numpy as np
 import pytest
 
@@ -35,21 +37,31 @@ def random_state(N, seed):
     return tuple(rng.standard_normal(s) for s in state_shapes(N))
 
 
-@pytest.mark.parametrize("precision,cfg", CFGS)
-@pytest.mark.parametrize("N", [8, 9, 10, 11, 16, 21, 23, 24, 31, 32, 33, 34, 46, 48, 65, 79])
-def test_apply_matches_oracle(precision, cfg, N):
-    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator
+AXIS = (0.3, -0.5, 0.8)
+
+
+@functools.lru_cache(maxsize=None)
+def linear_reference(N):
+    """A random state and the oracle's tendency, shared by the configurations."""
     from oracle.oracle import Oracle
-    h, u, v = random_state(N, 900 + N)
-    axis = (0.3, -0.5, 0.8)
-    ref = Oracle(N, h_mean=1000.0, axis=axis).apply(h, u, v)
-    dom = create_domain(N, precision=precision, h_mean=1000.0, rotation_axis=axis)
-    if cfg[1] == 1 and N <= 24:
-        # a block that touches four sides does not fit the register file with these configurations
-        try:
+    state = random_state(N, 900 + N)
+    return state, Oracle(N, h_mean=1000.0, axis=AXIS).apply(*state)
+
+
+@pytest.mark.parametrize("precision,cfg", CFGS)
+@pytest.mark.parametrize("N", [8, 9, 10, 11, 16, 21, 23, 24, 31, 32, 33, 34, 46, 48, 65, 79, 150])
+def test_apply_matches_oracle(precision, cfg, N):
+    """Up to more blocks than the device takes at once (C150).  FP64 configurations whose
+    blocks touch too many sides for the register file are refused: all of them where one tile
+    spans the panel both ways, the largest also where one spans it in one direction."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator
+    (h, u, v), ref = linear_reference(N)
+    dom = create_domain(N, precision=precision, h_mean=1000.0, rotation_axis=AXIS)
+    if precision == "fp64" and (N <= 11 or (cfg == (33, 1, 3) and N <= 24)):
+        with pytest.raises(SweError):
             dom.kernel_config = cfg
-        except SweError:
-            return
+        dom.destroy()
+        return
     dom.kernel_config = cfg
     assert dom.kernel_config == cfg
     op = create_swm_operator(dom.grav, LIN, dom)
@@ -134,11 +146,7 @@ def test_advective_apply_matches_oracle(precision, cfg, N, orography):
         o.set_orography(hs)
     ref = o.apply(h, u, v)
     dom = create_domain(N, precision=precision, rotation_axis=axis, operator="advective")
-    try:
-        dom.kernel_config = cfg
-    except SweError:
-        assert cfg[1] == 1 and N <= 24
-        return
+    dom.kernel_config = cfg
     assert dom.kernel_config == cfg
     op = create_swm_operator(dom.grav, {"swm_operator_type": "advective_swm_operator"}, dom)
     if orography:
@@ -218,4 +226,35 @@ def test_default_configuration(operator, precision, N, members, cfg):
     from ch_swe_b200 import create_domain
     dom = create_domain(N, precision=precision, n_members=members, operator=operator)
     assert dom.kernel_config == cfg
+    dom.destroy()
+
+
+@pytest.mark.parametrize("orography", [False, True])
+@pytest.mark.parametrize("precision,cfg", ADV_CFGS)
+def test_advective_members_of_every_configuration(precision, cfg, orography):
+    """RK4 steps of three members (own time steps, one frozen) with several tiles per direction,
+    against the oracle: the RK modes, the FP32 update's compensation and the FP32 tendencies."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    from oracle.oracle import Oracle
+    N, M = 66, 3
+    states = [random_state(N, 800 + k) for k in range(M)]
+    stack = [np.stack([s[f] + (0.0 if f else 1000.0) for s in states]) for f in range(3)]
+    dts = np.array([30.0, 0.0, 15.0])
+    hs = 100.0 * np.random.default_rng(9).standard_normal(stack[0][0].shape) if orography else None
+    dom = create_domain(N, precision=precision, n_members=M, operator="advective")
+    dom.kernel_config = cfg
+    op = create_swm_operator(dom.grav, {"swm_operator_type": "advective_swm_operator"}, dom)
+    o = Oracle(N, operator="advective")
+    if orography:
+        op.set_orography(hs)
+        o.set_orography(hs)
+    st = create_stvec_swm(dom).upload(*stack, member=None)
+    create_timescheme(st, "rk4").steps_members(st, op, dts, 3)
+    dom.synchronize()
+    out = st.download(member=None)
+    for m in (0, 2):
+        for g, r, name in zip(out, o.rk4(*(f[m] for f in stack), dts[m], 3), "huv"):
+            assert rel(g[m], r) < RTOL[precision], (m, name, rel(g[m], r))
+    for f in range(3):
+        assert np.array_equal(out[f][1], stack[f][1].astype(np.float32 if precision == "fp32" else np.float64))
     dom.destroy()
