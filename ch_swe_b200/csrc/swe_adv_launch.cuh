@@ -20,8 +20,10 @@ struct AdvOneTU {
                     const T *fmet, const double *dtm, int *err, cudaStream_t st);
     static void flux(int members, const T *y, const T *w, T *f, const Dims &d, const AdvView<T> &av, const MetricView<T> &m,
                      const double *dtm, cudaStream_t st);
-    // FP32 only: in FP64 the tiled k_advt is the faster one (C96 / C384 per RK4 step: 102 / 475 us
-    // against 108 / 499 us; in FP32 C96 / C384 95 / 315 against 89 / 278 us); false: not launched
+    // FP32 only (C96 / C384 per RK4 step 82 / 252 us; with k_advt 89 / 278 and 95 / 315 at older tile
+    // shapes).  FP64 runs the tiled k_advt; k_adv_tend there, measured at the present shapes: C48 73.5
+    // against 75.2 us, C96 81.8 / 86.6, C128 124 / 139, C192 163 / 164, C256 226 / 222, C384 411 / 405, 16 x
+    // C48 260 / 270: faster below C192, slower above.  false: not launched
     static bool tend(int label, int occ, int members, const CUtensorMap &tmY, const CUtensorMap &tmW, const T *vh, T *adt,
                      const Dims &d, const AdvView<T> &av, const OneMetric<T> &om, T inv_hxa, const double *dtm, int *err,
                      cudaStream_t st);

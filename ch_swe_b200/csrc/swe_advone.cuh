@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(TendLayout<T, XL, TH>::NM, 2)
                T *__restrict__ A, Dims d, AdvView<T> av, OneMetric<T> om, T inv_hxa, OneTiles ot, const double *__restrict__ dtm,
                int *err)
 {
+    static_assert(sizeof(T) == 4, "FP64 tendencies: k_advt (AdvOneTU::tend)");
     using C = TendLayout<T, XL, TH>;
     using L = OneLayout<T, XL, TH>;
     using V = OV<T>;
@@ -346,19 +347,10 @@ __global__ void __launch_bounds__(TendLayout<T, XL, TH>::NM, 2)
     auto tend = [&](const T *f, const V &a, const V &b) {
         T x[VW + 6];
         {
-            T lo[VW == 4 ? 4 : 4], hi[4];
-            if constexpr (VW == 4) {
-                const V l = ov_ld(f - 4), r = ov_ld(f + 4);
-#pragma unroll
-                for (int e = 0; e < 4; e++) { lo[e] = l.a[e]; hi[e] = r.a[e]; }
-            } else {
-                const V l0 = ov_ld(f - 4), l1 = ov_ld(f - 2), r0 = ov_ld(f + 2), r1 = ov_ld(f + 4);
-                lo[0] = l0.a[0]; lo[1] = l0.a[1]; lo[2] = l1.a[0]; lo[3] = l1.a[1];
-                hi[0] = r0.a[0]; hi[1] = r0.a[1]; hi[2] = r1.a[0]; hi[3] = r1.a[1];
-            }
+            const V l = ov_ld(f - 4), h = ov_ld(f + 4);
             const V c = ov_ld(f);
 #pragma unroll
-            for (int e = 0; e < 3; e++) { x[e] = lo[e + 1]; x[VW + 3 + e] = hi[e]; }
+            for (int e = 0; e < 3; e++) { x[e] = l.a[e + 1]; x[VW + 3 + e] = h.a[e]; }
 #pragma unroll
             for (int e = 0; e < VW; e++) x[3 + e] = c.a[e];
         }

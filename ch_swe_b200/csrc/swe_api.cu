@@ -1146,7 +1146,6 @@ static cudaError_t stage_smem_optin();
 //   Advective FP32: (33, 2), but (25, 2), 13 vectors by 18 rows, for one cube that two such tiles
 //   span; with (25, 2) / (33, 2): C52 74 / 73, C56 66 / 78, C64 70 / 87, C80 93 / 108, C96 82 / 85,
 //   C104 81 / 79, C192 103 / 97, 4 x C64 112 / 109, 16 x C80 333 / 293.
-constexpr int ONE_WAVE = 148;   // blocks of a kernel that takes an SM each
 template <class T>
 static KernelCfg one_default_cfg(int N, int members, bool adv)
 {

@@ -87,6 +87,8 @@ struct OneGrid {
     int sides;   // panel sides a tile can touch
 };
 
+constexpr int ONE_WAVE = 148;   // SMs: blocks of a kernel that takes an SM each
+
 // Tiles of at most XL - 2 HV vectors by TH rows, balanced.  The rows per tile are the
 // division with the least work on the busiest SM: blocks per SM times (rows + 6), the
 // window rows that the widest pass computes.  A panel with several tiles per direction
@@ -102,10 +104,10 @@ static inline bool one_grid(int N, int members, int xl, int th, int occ, OneGrid
     long long cost = 0;
     for (int gy = (n + th - 1) / th; gy <= n; gy++) {
         if (gy > 1 && n / gy < 7) break;
-        const long long blocks = (long long)gx * gy * NPAN * members, per = (blocks + 147) / 148;
+        const long long blocks = (long long)gx * gy * NPAN * members, per = (blocks + ONE_WAVE - 1) / ONE_WAVE;
         const long long c = per * ((n + gy - 1) / gy + 6);
         if (!best || c < cost) { best = gy; cost = c; }
-        if (blocks > 148LL * occ * 8) break;
+        if (blocks > 8LL * ONE_WAVE * occ) break;
     }
     if (!best) return false;
     og.g = dim3(gx, best, NPAN * members);

@@ -371,7 +371,7 @@ __global__ void __maxnreg__(REGS)
         const int s2 = lr ? (al == 1 ? SIDE_B : SIDE_T) : SIDE_L;
         T sn2 = T(0), sgx = T(0), sgy = T(0);
         bool y1 = false, y21 = false;
-        if (corner && lr && b < ONE_BAND) {
+        if (corner && lr) {
             const Link K2 = c_link[t][s2];
             const int kc = s == SIDE_L ? 1 : n, y2 = K2.rev ? n + 1 - kc : kc;
             y1 = y == 1;
