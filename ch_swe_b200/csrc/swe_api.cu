@@ -2445,7 +2445,7 @@ template <class T, int ORD, bool VEC>
 static void launch_laplacian(swe_ctx *c, const DifSplit &sp, const T *src, T *D1X, T *D1Y, T *R, T *dst, const AhView<T> &av,
                              const DifView<T> &dv)
 {
-    const int co = dif_carveout(c->cfg.N, c->cfg.n_members);
+    const int co = dif_carveout<T>(c->cfg.N, c->cfg.n_members, ORD);
     const dim3 g(DIF_HALF * (sp.ne + sp.ni), 1, NPAN * c->cfg.n_members * (DIF_FIELDS / DIF_HALF)), b(DIF_NT);
     launch_carveout(co, k_dif_d1<T, ORD, VEC>, g, b, 0, c->stream, src, D1X, D1Y, c->dims, av, sp);
     launch_carveout(co, k_dif_lap<T, ORD, VEC>, g, b, 0, c->stream, src, (const T *)D1X, (const T *)D1Y, R, dst, c->dims, av, dv, sp);
@@ -2466,7 +2466,7 @@ static int enqueue_diffusion(swe_ctx *c, T *y, T *out, double dt, const double *
 {
     int rc = dif_setup<T>(c);
     if (rc) return rc;
-    const int N = c->cfg.N, n = N + 1, M = c->cfg.n_members, co = dif_carveout(N, M);
+    const int N = c->cfg.N, n = N + 1, M = c->cfg.n_members, co = dif_carveout<T>(N, M, lap_order);
     const Dims d = c->dims;
     const size_t set = (size_t)M * DIF_FIELDS * NPAN * d.ps;
     T *X = (T *)c->dif, *D1X = X + set, *D1Y = X + 2 * set, *R = X + 3 * set, *A = X + 4 * set;

@@ -194,8 +194,12 @@ constexpr int DIF_NT = 128, DIF_HALF = 2;
 // Blocks per SM that k_dif_lap's registers leave room for.  Without vectors the kernels are
 // instantiations of their own: few enough registers that the next launch's blocks fit beside
 // them and start early.
+// (FP64 4-2 with 5 / 6: C256 249 / 254 us per RK4 step alone, 194 / 199 with three contexts.)
 template <class T>
-__host__ __device__ constexpr int dif_minb(int ord, bool vec) { return !vec ? 10 : (sizeof(T) == 4 && ord != 21 ? 8 : 6); }
+__host__ __device__ constexpr int dif_minb(int ord, bool vec)
+{
+    return !vec ? 10 : (sizeof(T) == 4 ? (ord == 21 ? 6 : 8) : (ord == 42 ? 5 : 6));
+}
 // Vertices of all fields from which on the interior goes by vectors (never in FP64 6-3, whose
 // vectors of two points read as many words as they save) and the diffusion's launches ask for
 // little shared memory (dif_carveout).  us per RK4 step with diffusion, alone, vectors / single
@@ -211,10 +215,19 @@ __host__ __device__ constexpr int dif_minb(int ord, bool vec) { return !vec ? 10
 constexpr long long DIF_LARGE = 200000;
 template <class T>
 __host__ __device__ constexpr bool dif_vectors(int ord) { return sizeof(T) == 4 || ord != 63; }
-static inline bool dif_large(int N, int members) { return (long long)(N + 1) * (N + 1) * NPAN * DIF_FIELDS * members >= DIF_LARGE; }
+static inline long long dif_vertices(int N, int members) { return (long long)(N + 1) * (N + 1) * NPAN * DIF_FIELDS * members; }
+static inline bool dif_large(int N, int members) { return dif_vertices(N, members) >= DIF_LARGE; }
 // Percent of the SM's L1 as shared memory, which the diffusion's kernels do not use: one value
-// for all of its launches, so that no SM drains to change it between them.
-static inline int dif_carveout(int N, int members) { return dif_large(N, members) ? 8 : cudaSharedmemCarveoutDefault; }
+// for all of its launches, so that no SM drains to change it between them.  Not in FP32 2-1 and
+// 4-2 from C145 on: contexts beside one another lose more than one alone gains there (C192 4-2 with
+// / without: alone 127 / 135 us per RK4 step, three contexts 82.6 / 79.0; C96 95.6 / 100 and 40.4 /
+// 44.4; C192 6-3 184.7 / 191.3 and 106.5 / 111.2; C192 FP64 4-2 180.2 / 183.0 and 123.8 / 128.1).
+template <class T>
+static inline int dif_carveout(int N, int members, int ord)
+{
+    const bool most = sizeof(T) == 4 && ord != 63 && dif_vertices(N, members) >= 500000;
+    return dif_large(N, members) && !most ? 8 : cudaSharedmemCarveoutDefault;
+}
 
 // Split of a panel's n x n vertices for the difference passes: the vectors (swe_vec.cuh)
 // whose points and rows all take interior rows of both the narrow second difference and the
