@@ -10,9 +10,10 @@
 // components and flux beside the edge itself, so the stage needs no edge strips and no
 // edge-sync launch; k_advhalo (swe_advective.cuh) is shared with the split stage.
 //
-// Measured at C384 FP32 per launch (B200, cold L2, ncu): k_co2contra 22.8 -> k_adv_co2 10.6 us,
-// k_stage 55.2 -> k_adv_stage 27 us, k_advt 27.8 -> k_adv_tend 17.8 us, k_edge 6.0 us and its
-// strips gone; an RK4 step alone 444 -> 222 us.  The kernels wait for memory latency between
+// Measured at C384 FP32 per launch (B200, cold L2, ncu): k_co2contra 22.8 -> k_adv_co2 9.8 us,
+// k_stage 55.2 -> k_adv_stage 24.8 us, k_advt 27.8 -> k_adv_tend 15.2 us, k_edge 6.0 us and its
+// strips gone; an RK4 step alone 444 us autotuned -> 252 (33, 2) or 220 (25, 2), with three
+// contexts beside one another 367 -> 176.  The kernels wait for memory latency between
 // short passes (the stage's windows and metric are nine TMA boxes per tile; the flux reads
 // seven vectors per thread): more bytes in flight, not fewer operations, would shorten them.
 #pragma once

@@ -219,7 +219,7 @@ static inline long long dif_vertices(int N, int members) { return (long long)(N 
 static inline bool dif_large(int N, int members) { return dif_vertices(N, members) >= DIF_LARGE; }
 // Percent of the SM's L1 as shared memory, which the diffusion's kernels do not use: one value
 // for all of its launches, so that no SM drains to change it between them.  Not in FP32 2-1 and
-// 4-2 from C145 on: contexts beside one another lose more than one alone gains there (C192 4-2 with
+// 4-2 from C144 on: contexts beside one another lose more than one alone gains there (C192 4-2 with
 // / without: alone 127 / 135 us per RK4 step, three contexts 82.6 / 79.0; C96 95.6 / 100 and 40.4 /
 // 44.4; C192 6-3 184.7 / 191.3 and 106.5 / 111.2; C192 FP64 4-2 180.2 / 183.0 and 123.8 / 128.1).
 template <class T>

@@ -28,9 +28,9 @@
 // per block, two rows per thread and the boundary as a loop of the same threads ran 17 us per
 // stage even at C24: the boundary's chain of dependent loads stood in the passes' way; its
 // threads of their own brought C24 to 6 us.  A stage's time now is one memory round trip for the
-// windows (0.8 us), four passes of 0.4 to 0.9 us and the RK4 stores; ncu counts 22 % of the L2
-// and 62 % of the shared-memory throughput at C384, issue slots 35 to 45 % busy: latency and
-// shared-memory traffic, not arithmetic (three instead of four operations per stencil and
+// windows (0.8 us), four passes of 0.4 to 0.9 us and the RK4 stores; ncu counts 21 % of the L2
+// throughput, 58 % of the L1's and 39 % of the shared-memory wavefronts at C384, issue slots 36 %
+// busy: latency and shared-memory traffic, not arithmetic (three instead of four operations per stencil and
 // packed FP32 changed nothing at C192).  Assigning the vectors of a pass to threads one after
 // another, without idle lanes, saved 14 % of the instructions and ran 5 to 25 % slower: the
 // rows' ends conflict in shared memory and fewer warps hide the latency.
