@@ -1303,6 +1303,8 @@ extern "C" int swe_synchronize(swe_ctx *c)
     if (!c) return SWE_EINVAL;
     const int rc = results_ready(c);
     *c->derr = 0;
+    // and the default stream, where a host program may have written a state through its device view
+    CU(c, cudaStreamSynchronize(cudaStreamLegacy));
     return rc;
 }
 

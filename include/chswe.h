@@ -103,7 +103,7 @@ int swe_ctx_destroy(swe_ctx *ctx);
 const char *swe_last_error(const swe_ctx *ctx);
 /* Run the context's work on an existing CUDA stream (cudaStream_t); NULL restores the own stream. */
 int swe_set_stream(swe_ctx *ctx, void *cuda_stream);
-/* Wait for the context's work.  SWE_ECUDA after a stage kernel whose tile loads did not arrive
+/* Wait for the context's work and for the default stream's.  SWE_ECUDA after a stage kernel whose tile loads did not arrive
    within a second: the states it wrote are incomplete.  Until swe_synchronize has reported it,
    every call that returns results to the host (downloads, integrals, diagnostics, lat-lon
    regrids, kernel times) returns the same error. */

@@ -102,3 +102,28 @@ def test_tables_of_the_diagnostics_on_first_use(N, what):
         dom.destroy()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_synchronize_waits_for_the_default_stream():
+    """A state written through its device view by work on the default stream is in place after
+    swe_synchronize, for the context's stream."""
+    import math
+    import torch
+    ic, dom, _, st = make(16, idle)
+    ptr, nbytes, _, _ = st.device_view()
+
+    class View:
+        __cuda_array_interface__ = {"data": (ptr, False), "shape": (nbytes // 8,), "typestr": "<f8", "version": 3}
+
+    box = torch.as_tensor(View(), device="cuda")
+    assert math.prod(box.shape) * 8 == nbytes
+    box.mul_(1.0)   # the kernel is loaded
+    idle()
+    busy()
+    box.mul_(2.0)
+    dom.synchronize()
+    for a, b in zip(ic, st.download()):
+        assert np.array_equal(2.0 * a, b)
+    idle()
+    del box, st
+    dom.destroy()
