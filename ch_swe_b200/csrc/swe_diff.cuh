@@ -412,9 +412,12 @@ __global__ void __launch_bounds__(DIF_NT, dif_minb<T>(ORD, VEC)) k_dif_lap(
         }
 #pragma unroll
         for (int e = 0; e < VW; e++) {
-            T d2x = wx[0].a[e] * x[e], d2y = wy[0].a[e] * y[0].a[e], c[2 * R + 1];
+            // narrow_d2's order of summation: a vertex has the same bits either way
+            constexpr int M0 = ORD == 21 ? 2 * R : 0, DM = ORD == 21 ? -1 : 1;
+            T d2x = wx[M0].a[e] * x[e + M0], d2y = wy[M0].a[e] * y[M0].a[e], c[2 * R + 1];
 #pragma unroll
-            for (int m = 1; m < 2 * R + 1; m++) {
+            for (int q = 1; q < 2 * R + 1; q++) {
+                const int m = M0 + DM * q;
                 d2x = d2x + wx[m].a[e] * x[e + m];
                 d2y = d2y + wy[m].a[e] * y[m].a[e];
             }

@@ -93,6 +93,27 @@ def test_apply_parity_of_vectors_and_single_vertices(order, N, precision):
     dom.destroy()
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("order", [21, 42, 63])
+def test_members_have_the_bits_of_single_contexts(order, precision):
+    """C40: eight members go by vectors, one member by single vertices; the same bits."""
+    from ch_swe_b200 import create_stvec_swm, create_swm_diff_operator
+    N, M = 40, 8
+    states = [random_state(N, 60 + m) for m in range(M)]
+    out = []
+    for members in (M, 1):
+        dom, _ = ah_domain(N, precision, members=members)
+        dif = create_swm_diff_operator(diff_config(order), dom)
+        x, y = create_stvec_swm(dom), create_stvec_swm(dom)
+        for m in range(members):
+            x.upload(*states[5 if members == 1 else m], member=m)
+        dif.apply(y, x, dom)
+        out.append(y.download(member=5 if members > 1 else 0))
+        dom.destroy()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("order", [21, 42, 63])
 def test_euler_steps_and_driver_loop_fp64(order):
     """Six driver steps on a Gaussian hill: RK4 of the Ah linear operator of the same SBP
