@@ -53,8 +53,8 @@ bool OneTU<T>::grid(int label, int occ, int N, int members, OneGrid &g)
 {
 #define CHSWE_O(LABEL, XL, TH, OCC, REGS)  \
     if (label == LABEL && occ == OCC)      \
-        return one_grid<T>(N, members, XL, TH, OCC, g) &&  \
-               one_fits((OneLayout<T, XL, TH>::NM + g.sides * ONE_BAND) / 32, REGS);
+        return one_grid<T>(N, members, XL, TH, OCC,        \
+                           [](int sides) { return one_fits((OneLayout<T, XL, TH>::NM + sides * ONE_BAND) / 32, REGS); }, g);
     CHSWE_ONE_EACH(CHSWE_O)
 #undef CHSWE_O
     return false;

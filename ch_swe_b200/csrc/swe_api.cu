@@ -1124,8 +1124,9 @@ template <class T>
 static cudaError_t stage_smem_optin();
 
 // The vector stage's configuration a Ch 4-2 context starts with; tile 0: the split kernels, where
-// no tile of the configuration fits the register file (blocks that touch four sides: linear FP64
-// below C13, and some larger member counts up to C16).  Small cubes, linear, alone, split /
+// no tile of a configuration fits the register file (blocks that touch four sides: linear FP64
+// below C13).  The cube alone decides between the two, and every tile shape gives the same bits:
+// a member of an ensemble has those of a context of its own.  Small cubes, linear, alone, split /
 // vector, us per RK4 step: C8 FP32 61 / 19, C15 FP32 65 / 19, C15 FP64 71 / 20.
 // us per RK4 step, alone:
 //   Linear FP32: tiles of 7 vectors by 28 rows at every size (C48 / C96 / C192 / C384 19.9 / 22.6 /
@@ -1133,9 +1134,10 @@ static cudaError_t stage_smem_optin();
 //   576 against 1139).
 //   Linear FP64: full-width tiles for several members of a cube that one tile spans (64 x C48
 //   305 against 389 with (25, 1), 351 with (33, 1) and 448 split: fewer panel corners per block).
-//   Below C26 only while the panels make one wave: beyond it (25, 1), where it fits (64 x C24 157
-//   / 195 / 184 with (25, 1) / (17, 1) / split), else split from two waves on (128 x C18 330 /
-//   260 with (17, 1) / split, 16 x C18 58 / 85).  A few members of larger cubes: tiles of 10
+//   Below C26 only for up to 16 members of C20 and more, else (25, 1); with (17, 1) / (25, 1) / split:
+//   8 x C18 30 / 23 / 82, 128 x C18 330 / 241 / 260, 8 x C22 31 / 42 / 85, 16 x C22 59 / 64 / 91, 24 x
+//   C22 66 / 53 / 91, 64 x C24 195 / 157 / 184, 64 x C26 198 / 233 / 286; 256 x C13 599 / 448 / 426, the
+//   one range where split is the faster.  A few members of larger cubes: tiles of 10
 //   vectors by 25 rows where they make at most one wave (C96: 27.4 against 29.0), else 14 vectors by
 //   28 rows (C192 69 against 102 split, C384 213 against 265 fused).
 //   Advective FP64: (25, 2) for several members of small cubes, otherwise the largest tiles,
@@ -1159,11 +1161,9 @@ static KernelCfg one_default_cfg(int N, int members, bool adv)
         return AdvOneTU<T>::grid(k.tile, k.occ, N, members, og) ? k : none;
     }
     if (sizeof(T) == 4) return OneTU<T>::grid(33, 2, N, members, og) ? KernelCfg{33, 2, 3} : none;
-    if (members > 4 && OneTU<T>::grid(17, 1, N, members, og) && og.g.x == 1) {
-        if (N >= 26 || NPAN * members <= ONE_WAVE) return KernelCfg{17, 1, 3};
-        if (OneTU<T>::grid(25, 1, N, members, og)) return KernelCfg{25, 1, 3};
-        return NPAN * members <= 2 * ONE_WAVE ? KernelCfg{17, 1, 3} : none;
-    }
+    if (members > 4 && (N >= 26 || (N >= 20 && members <= 16)) && OneTU<T>::grid(17, 1, N, members, og) && og.g.x == 1)
+        return KernelCfg{17, 1, 3};
+    if (N < 26) return OneTU<T>::grid(25, 1, N, members, og) ? KernelCfg{25, 1, 3} : none;
     for (int label : {25, 33})
         if (OneTU<T>::grid(label, 1, N, members, og) && (blocks() <= ONE_WAVE || label == 33)) return KernelCfg{label, 1, 3};
     return none;

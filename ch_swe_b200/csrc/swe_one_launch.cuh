@@ -92,9 +92,11 @@ constexpr int ONE_WAVE = 148;   // SMs: blocks of a kernel that takes an SM each
 // Tiles of at most XL - 2 HV vectors by TH rows, balanced.  The rows per tile are the
 // division with the least work on the busiest SM: blocks per SM times (rows + 6), the
 // window rows that the widest pass computes.  A panel with several tiles per direction
-// needs seven points in each of them.
-template <class T>
-static inline bool one_grid(int N, int members, int xl, int th, int occ, OneGrid &og)
+// needs seven points in each of them.  fits(sides): whether a block with the band threads of that
+// many panel sides fits the register file; a division whose blocks do not is passed over, so that
+// the cube, not the number of its members, decides whether a configuration is available.
+template <class T, class Fits>
+static inline bool one_grid(int N, int members, int xl, int th, int occ, const Fits &fits, OneGrid &og)
 {
     constexpr int VW = OV<T>::W, HV = 4 / VW;
     const int n = N + 1, nv = (n + VW - 1) / VW, wv = xl - 2 * HV;
@@ -106,8 +108,8 @@ static inline bool one_grid(int N, int members, int xl, int th, int occ, OneGrid
         if (gy > 1 && n / gy < 7) break;
         const long long blocks = (long long)gx * gy * NPAN * members, per = (blocks + ONE_WAVE - 1) / ONE_WAVE;
         const long long c = per * ((n + gy - 1) / gy + 6);
-        if (!best || c < cost) { best = gy; cost = c; }
-        if (blocks > 8LL * ONE_WAVE * occ) break;
+        if (fits((gx == 1 ? 2 : 1) + (gy == 1 ? 2 : 1)) && (!best || c < cost)) { best = gy; cost = c; }
+        if (best && blocks > 8LL * ONE_WAVE * occ) break;
     }
     if (!best) return false;
     og.g = dim3(gx, best, NPAN * members);

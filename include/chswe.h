@@ -294,7 +294,7 @@ int swe_get_tile(const swe_ctx *ctx, int *tile);
    (33, 2, 0).  The advective operator's stage kernel always uses the tile's first
    blocks-per-SM value.  runs 2: the fused stage (linear operator, Ch, SBP 4-2).  runs 3:
    the vector stage of Ch contexts in SBP 4-2, the default where one of its tiles suits
-   the cube (linear FP64: from 13 cells on, with some exceptions below 26) -- linear
+   the cube (all but linear FP64 below 13 cells, whatever the members) -- linear
    operator one launch per RK stage, advective five; tile is at least the rows of its
    tiles.  Linear FP32 (17, 2), (25, 2), (33, 2), FP64 (17, 1), (25, 1), (33, 1);
    advective FP32 (25, 2), (33, 2), FP64 (17, 2), (25, 2), (33, 1); a configuration that

@@ -215,14 +215,14 @@ def test_default_stage_of_the_smallest_cubes(N, operator, precision):
 
 
 @pytest.mark.parametrize("operator,precision,N,members,cfg", [
-    ("linear", "fp64", 18, 16, (17, 1, 3)), ("linear", "fp64", 18, 64, (25, 2, 0)), ("linear", "fp64", 24, 64, (25, 1, 3)),
+    ("linear", "fp64", 18, 16, (25, 1, 3)), ("linear", "fp64", 22, 16, (17, 1, 3)), ("linear", "fp64", 22, 24, (25, 1, 3)), ("linear", "fp64", 18, 64, (25, 1, 3)), ("linear", "fp64", 12, 64, (25, 2, 0)), ("linear", "fp64", 24, 64, (25, 1, 3)),
     ("linear", "fp64", 26, 64, (17, 1, 3)), ("linear", "fp64", 96, 1, (25, 1, 3)), ("linear", "fp64", 192, 1, (33, 1, 3)),
     ("linear", "fp32", 192, 1, (33, 2, 3)), ("advective", "fp64", 108, 1, (33, 1, 3)), ("advective", "fp64", 128, 1, (17, 2, 3)),
     ("advective", "fp64", 64, 4, (25, 2, 3)), ("advective", "fp64", 80, 16, (17, 2, 3)), ("advective", "fp32", 52, 1, (33, 2, 3)), ("advective", "fp32", 80, 1, (25, 2, 3)),
     ("advective", "fp32", 80, 4, (33, 2, 3)), ("advective", "fp32", 128, 1, (33, 2, 3))])
 def test_default_configuration(operator, precision, N, members, cfg):
     """The configuration a context starts with, on both sides of each line of the rule: the
-    sizes at which another one was measured slower than the split kernels are among them."""
+    sizes at which another one was measured slower are among them."""
     from ch_swe_b200 import create_domain
     dom = create_domain(N, precision=precision, n_members=members, operator=operator)
     assert dom.kernel_config == cfg
@@ -258,3 +258,26 @@ def test_advective_members_of_every_configuration(precision, cfg, orography):
     for f in range(3):
         assert np.array_equal(out[f][1], stack[f][1].astype(np.float32 if precision == "fp32" else np.float64))
     dom.destroy()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("N,members", [(12, 16), (13, 16), (14, 64), (16, 16), (16, 64), (18, 128), (24, 64), (30, 48)])
+def test_members_have_the_bits_of_single_contexts(N, members, precision):
+    """Whether a cube starts on the vector stage does not depend on its number of members, and
+    every tile shape gives the same bits: a member's are those of a context of its own."""
+    from ch_swe_b200 import create_domain, create_stvec_swm, create_swm_operator, create_timescheme
+    states = [random_state(N, 20 + k) for k in range(3)]
+    picked = {0: 0, members // 2: 1, members - 1: 2}
+    out = []
+    for M in (members, 1, 1, 1):
+        dom = create_domain(N, precision=precision, n_members=M, h_mean=1000.0)
+        op = create_swm_operator(dom.grav, LIN, dom)
+        st = create_stvec_swm(dom)
+        for m, k in picked.items() if M > 1 else ((0, len(out) - 1),):
+            st.upload(*states[k], member=m)
+        create_timescheme(st, "rk4").steps(st, op, dom, 100.0, 3)
+        out.append([st.download(member=m) for m in (picked if M > 1 else (0,))])
+        dom.destroy()
+    for k in range(3):
+        for a, b in zip(out[0][k], out[1 + k][0]):
+            assert np.array_equal(a, b)
