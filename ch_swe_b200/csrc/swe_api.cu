@@ -1142,9 +1142,10 @@ static cudaError_t stage_smem_optin();
 //   28 rows (C192 69 against 102 split, C384 213 against 265 fused).
 //   Advective FP64: (25, 2) for several members of small cubes, otherwise the largest tiles,
 //   (33, 1), where they make at most one wave, else (17, 2); with (17, 2) / (25, 2) / (33, 1): 16 x
-//   C36 208 / 190 / 217, 4 x C64 170 / 158 / 169, 4 x C96 209 / 211 / 260, one cube C48 77 / 77 / 75, C96 94 / 94 / 86, C108 89 / 94 / 81, C112 106 /
-//   108 / 152, C128 138 / 164 / 177, C144 174 / 173 / 165, C160 179 / 152 / 187, C192 164 / 166 / 189, C256 223 / 221 / 255,
-//   C384 405 / 455 / 459, 16 x C80 443 / 486 / 453.
+//   C36 208 / 190 / 217, 4 x C64 170 / 158 / 169, 4 x C96 209 / 211 / 260, 16 x C80 443 / 486 / 453; one
+//   cube C48 77 / 77 / 75, C96 94 / 94 / 86, C108 89 / 94 / 81, C112 106 / 108 / 152, C128 138 / 164 / 177,
+//   C144 174 / 173 / 165, C160 179 / 152 / 187, C192 164 / 166 / 189, C256 223 / 221 / 255, C384 405 /
+//   455 / 459.
 //   Advective FP32: (33, 2), but (25, 2), 13 vectors by 18 rows, for one cube that two such tiles
 //   span; with (25, 2) / (33, 2): C52 74 / 73, C56 66 / 78, C64 70 / 87, C80 93 / 108, C96 82 / 85,
 //   C104 81 / 79, C192 103 / 97, 4 x C64 112 / 109, 16 x C80 333 / 293.
